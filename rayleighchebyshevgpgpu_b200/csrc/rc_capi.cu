@@ -510,9 +510,7 @@ rc_status rc_rayleigh_ritz(rc_ctx* ctx, const rc_op* op_c, void* V, void* W, int
     const int dt = op->dtype;
     const size_t esz = elem_bytes(dt, P64);
     const int64_t n = op->n;
-    void *T1 = nullptr, *T2 = nullptr, *sm = nullptr;
-    RC_TRY(rc_slot(ctx, S_T1, (size_t)n * s * esz, &T1));
-    RC_TRY(rc_slot(ctx, S_T2, (size_t)n * s * esz, &T2));
+    void* sm = nullptr;
     const size_t mat = (size_t)s * s * esz;
     RC_TRY(rc_slot(ctx, S_IO, 3 * mat + (size_t)s * 16 + 256, &sm));
     void* H = sm;
@@ -527,17 +525,38 @@ rc_status rc_rayleigh_ritz(rc_ctx* ctx, const rc_op* op_c, void* V, void* W, int
     RC_TRY(rcb::op_step(ctx, op, st));
     RC_TRY(rcb::gram(ctx, dt, n, s, s, V, ld, W, ld, H, true));
     RC_TRY(rcb::small_eigh(ctx, dt, s, H, Qd, dlam, dinfo));
-    rcb::XtArgs a;
-    a.n = n; a.k = s; a.nc = s;
-    a.X = V; a.ldx = ld;
-    a.T = Qd; a.ldt = s;
-    a.Y = T1; a.ldy = n;
-    a.X2 = W; a.ldx2 = ld;
-    a.Y2 = T2; a.ldy2 = n;
-    a.lam = dlam; a.res_count = res_count; a.res = dres;
-    RC_TRY(rcb::xt(ctx, dt, a));
-    RC_TRY(rcb::copy_cols(ctx, dt, T1, n, V, ld, n, s));
-    RC_TRY(rcb::copy_cols(ctx, dt, T2, n, W, ld, n, s));
+    if (op->kind != 2) {
+        // native operators: V <- V Q (in place where one pass holds the columns), then W <- A V once more and
+        // the residual norms from the two blocks. Against W Q formed beside V Q by one SIMT kernel, and both
+        // blocks copied back: 6.3 instead of 11.2 ms on the 128^3 CSR operator with 96 columns, 12.3 instead of
+        // 23.9 ms on a complex 7-point stencil with 442,368 rows and 192 columns (a sparse product costs 1.2
+        // and 0.9 ms there, a second dense one 1.2 and 3.8 ms).
+        if (rcb::xt_dmma_in_place(s)) {
+            RC_TRY(rcb::xt_dmma(ctx, dt, n, s, s, V, ld, false, Qd, s, V, ld));
+        } else {
+            void* T1 = nullptr;
+            RC_TRY(rc_slot(ctx, S_T1, (size_t)n * s * esz, &T1));
+            RC_TRY(rcb::xt_dmma(ctx, dt, n, s, s, V, ld, false, Qd, s, T1, n));
+            RC_TRY(rcb::copy_cols(ctx, dt, T1, n, V, ld, n, s));
+        }
+        RC_TRY(rcb::op_step(ctx, op, st));
+        RC_TRY(rcb::resid_norms(ctx, dt, n, res_count, V, ld, W, ld, dlam, dres));
+    } else {
+        void *T1 = nullptr, *T2 = nullptr;
+        RC_TRY(rc_slot(ctx, S_T1, (size_t)n * s * esz, &T1));
+        RC_TRY(rc_slot(ctx, S_T2, (size_t)n * s * esz, &T2));
+        rcb::XtArgs a;
+        a.n = n; a.k = s; a.nc = s;
+        a.X = V; a.ldx = ld;
+        a.T = Qd; a.ldt = s;
+        a.Y = T1; a.ldy = n;
+        a.X2 = W; a.ldx2 = ld;
+        a.Y2 = T2; a.ldy2 = n;
+        a.lam = dlam; a.res_count = res_count; a.res = dres;
+        RC_TRY(rcb::xt(ctx, dt, a));
+        RC_TRY(rcb::copy_cols(ctx, dt, T1, n, V, ld, n, s));
+        RC_TRY(rcb::copy_cols(ctx, dt, T2, n, W, ld, n, s));
+    }
     RC_CU(ctx, cudaMemcpyAsync(evals, dlam, s * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
     if (residuals && res_count > 0)
         RC_CU(ctx, cudaMemcpyAsync(residuals, dres, res_count * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));

@@ -151,10 +151,12 @@ rc_status gram(rc_ctx* ctx, int dtype, int64_t n, int64_t m, int64_t nc, const v
 }
 
 // ---------------------------------------------------------------------------------------
-// XT: Y = beta*Y + X*T  (X: n x k, T: k x nc, Y: n x nc), optional dual + residuals.
+// XT: Y = beta*Y + X*T  (X: n x k, T: k x nc, Y: n x nc) with a second pair Y2 = X2*T (stored unless Y2 is
+// null) and residuals, for callback operators, whose apply is not called again for A*(X*T). Plain products
+// are xt_dmma's (rc_xt.cu).
 // grid: (ceil(n/64), ceil(nc/64)); thread (tx,ty): rows r0 + tx + 16 i, cols c0 + ty + 16 j.
 // ---------------------------------------------------------------------------------------
-template <class T, bool DUAL>
+template <class T>
 __global__ void __launch_bounds__(TPB)
 xt_kernel(int64_t n, int64_t k, int64_t nc, const T* __restrict__ X, int64_t ldx, const T* __restrict__ Tm,
           int64_t ldt, T* __restrict__ Y, int64_t ldy, double alpha, double beta, const T* __restrict__ X2, int64_t ldx2,
@@ -163,20 +165,18 @@ xt_kernel(int64_t n, int64_t k, int64_t nc, const T* __restrict__ X, int64_t ldx
     constexpr int KX = IsComplex<T>::value ? 8 : 16;  // K-tile depth (complex: 48 KB static smem limit)
     const int64_t r0 = (int64_t)blockIdx.x * TB, c0 = (int64_t)blockIdx.y * TB;
     __shared__ T Xs[KX][TB + 1];
-    __shared__ T X2s[DUAL ? KX : 1][TB + 1];
+    __shared__ T X2s[KX][TB + 1];
     __shared__ T Ts[KX][TB + 1];
     const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
-    T acc[4][4], acc2[DUAL ? 4 : 1][DUAL ? 4 : 1];
+    T acc[4][4], acc2[4][4];
 #pragma unroll
     for (int i = 0; i < 4; ++i)
 #pragma unroll
         for (int j = 0; j < 4; ++j) acc[i][j] = s_zero(T());
-    if (DUAL) {
 #pragma unroll
-        for (int i = 0; i < (DUAL ? 4 : 1); ++i)
+    for (int i = 0; i < 4; ++i)
 #pragma unroll
-            for (int j = 0; j < (DUAL ? 4 : 1); ++j) acc2[i][j] = s_zero(T());
-    }
+        for (int j = 0; j < 4; ++j) acc2[i][j] = s_zero(T());
     for (int64_t k0 = 0; k0 < k; k0 += KX) {
         // X tile: 64 rows x KX cols; element e: rr = e % 64 (row), kk = e / 64
 #pragma unroll
@@ -186,7 +186,7 @@ xt_kernel(int64_t n, int64_t k, int64_t nc, const T* __restrict__ X, int64_t ldx
             const int64_t r = r0 + rr, kc = k0 + kk;
             const bool ok = r < n && kc < k;
             Xs[kk][rr] = ok ? X[r + kc * ldx] : s_zero(T());
-            if (DUAL) X2s[kk][rr] = ok ? X2[r + kc * ldx2] : s_zero(T());
+            X2s[kk][rr] = ok ? X2[r + kc * ldx2] : s_zero(T());
         }
         // T tile: KX rows x 64 cols; element e: kk = e % KX, cc = e / KX
 #pragma unroll
@@ -208,16 +208,14 @@ xt_kernel(int64_t n, int64_t k, int64_t nc, const T* __restrict__ X, int64_t ldx
             for (int i = 0; i < 4; ++i)
 #pragma unroll
                 for (int j = 0; j < 4; ++j) acc[i][j] = s_fma(a[i], b[j], acc[i][j]);
-            if (DUAL) {
-                T a2[4];
+            T a2[4];
 #pragma unroll
-                for (int i = 0; i < 4; ++i) a2[i] = X2s[kk][tx + 16 * i];
+            for (int i = 0; i < 4; ++i) a2[i] = X2s[kk][tx + 16 * i];
 #pragma unroll
-                for (int i = 0; i < 4; ++i)
+            for (int i = 0; i < 4; ++i)
 #pragma unroll
-                    for (int j = 0; j < 4; ++j) acc2[i % (DUAL ? 4 : 1)][j % (DUAL ? 4 : 1)] =
-                        s_fma(a2[i], b[j], acc2[i % (DUAL ? 4 : 1)][j % (DUAL ? 4 : 1)]);
-            }
+                for (int j = 0; j < 4; ++j) acc2[i][j] =
+                    s_fma(a2[i], b[j], acc2[i][j]);
         }
         __syncthreads();
     }
@@ -226,7 +224,7 @@ xt_kernel(int64_t n, int64_t k, int64_t nc, const T* __restrict__ X, int64_t ldx
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
         const int64_t c = c0 + ty + 16 * j;
-        const double lc = (DUAL && lam && c < res_count) ? lam[c] : 0.0;
+        const double lc = (lam && c < res_count) ? lam[c] : 0.0;
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
             const int64_t r = r0 + tx + 16 * i;
@@ -234,15 +232,13 @@ xt_kernel(int64_t n, int64_t k, int64_t nc, const T* __restrict__ X, int64_t ldx
                 T v = alpha == 1.0 ? acc[i][j] : s_rscale(alpha, acc[i][j]);
                 if (beta != 0.0) v = s_add(v, s_rscale(beta, Y[r + c * ldy]));
                 Y[r + c * ldy] = v;
-                if (DUAL) {
-                    const T w = acc2[i % (DUAL ? 4 : 1)][j % (DUAL ? 4 : 1)];
-                    if (Y2) Y2[r + c * ldy2] = w;
-                    if (lam && c < res_count) rs[j] += s_abs2(s_sub(w, s_rscale(lc, v)));
-                }
+                const T w = acc2[i][j];
+                if (Y2) Y2[r + c * ldy2] = w;
+                if (lam && c < res_count) rs[j] += s_abs2(s_sub(w, s_rscale(lc, v)));
             }
         }
     }
-    if (DUAL && lam) {
+    if (lam) {
         // reduce over tx (16 lanes of a half-warp share ty)
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
@@ -269,21 +265,15 @@ template <class T>
 static rc_status xt_t(rc_ctx* ctx, const XtArgs& a) {
     const unsigned gx = (unsigned)((a.n + TB - 1) / TB), gy = (unsigned)((a.nc + TB - 1) / TB);
     dim3 grid(gx, gy);
-    const bool dual = a.X2 != nullptr;
     double* rpart = nullptr;
-    if (dual && a.lam && a.res_count > 0) {
+    if (a.lam && a.res_count > 0) {
         void* p = nullptr;
         RC_TRY(rc_slot(ctx, S_RPART, (size_t)gx * a.res_count * sizeof(double), &p));
         rpart = (double*)p;
     }
-    if (dual)
-        xt_kernel<T, true><<<grid, TPB, 0, ctx->stream>>>(
-            a.n, a.k, a.nc, (const T*)a.X, a.ldx, (const T*)a.T, a.ldt, (T*)a.Y, a.ldy, a.alpha, a.beta, (const T*)a.X2,
-            a.ldx2, (T*)a.Y2, a.ldy2, rpart ? a.lam : nullptr, a.res_count, rpart);
-    else
-        xt_kernel<T, false><<<grid, TPB, 0, ctx->stream>>>(a.n, a.k, a.nc, (const T*)a.X, a.ldx, (const T*)a.T,
-                                                           a.ldt, (T*)a.Y, a.ldy, a.alpha, a.beta, nullptr, 0, nullptr, 0,
-                                                           nullptr, 0, nullptr);
+    xt_kernel<T><<<grid, TPB, 0, ctx->stream>>>(a.n, a.k, a.nc, (const T*)a.X, a.ldx, (const T*)a.T, a.ldt, (T*)a.Y,
+                                                a.ldy, a.alpha, a.beta, (const T*)a.X2, a.ldx2, (T*)a.Y2, a.ldy2,
+                                                rpart ? a.lam : nullptr, a.res_count, rpart);
     ctx->launches++;
     RC_CU(ctx, cudaGetLastError());
     if (rpart) {
@@ -296,16 +286,16 @@ static rc_status xt_t(rc_ctx* ctx, const XtArgs& a) {
 
 rc_status xt(rc_ctx* ctx, int dtype, const XtArgs& a) {
     if (a.n <= 0 || a.nc <= 0) return RC_OK;
-    // real fast path: plain products and residual-only dual products
-    const bool plain = a.alpha == 1.0 && a.beta == 0.0;
-    const bool dual_res_only =
-        a.X2 != nullptr && a.Y2 == nullptr && a.lam != nullptr && (a.res_count > 0 || a.R32 != nullptr);
-    if (plain && (a.X2 == nullptr || dual_res_only) && xt2_supported(dtype, a.k, a.nc))
+    if (a.X2 == nullptr)
+        return xt_dmma(ctx, dtype, a.n, a.k, a.nc, a.X, a.ldx, false, a.T, a.ldt, a.Y, a.ldy, a.alpha, a.beta, a.Yrm,
+                       a.ldyr);
+    // real fast path: residual-only dual products
+    const bool res_only = a.Y2 == nullptr && a.lam != nullptr && (a.res_count > 0 || a.R32 != nullptr);
+    if (a.alpha == 1.0 && a.beta == 0.0 && res_only && xt2_supported(dtype, a.k, a.nc))
         return xt2(ctx, a.n, a.k, a.nc, (const double*)a.X, a.ldx, (const double*)a.T, a.ldt, (double*)a.Y, a.ldy,
-                   (const double*)a.X2, a.ldx2, a.lam, dual_res_only ? a.res_count : 0, a.res, a.R32, a.ldr, a.Yrm,
-                   a.ldyr);
+                   (const double*)a.X2, a.ldx2, a.lam, a.res_count, a.res, a.R32, a.ldr);
     if (a.R32 || a.Yrm)
-        return rc_fail(ctx, RC_ERR_UNSUPPORTED, "xt: row-major outputs need a real block of <= 96 columns");
+        return rc_fail(ctx, RC_ERR_UNSUPPORTED, "xt: row-major outputs of a dual product need a real block of <= 96 columns");
     return dtype == RC_COMPLEX128 ? xt_t<double2>(ctx, a) : xt_t<double>(ctx, a);
 }
 

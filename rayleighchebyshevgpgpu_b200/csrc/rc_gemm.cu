@@ -9,10 +9,9 @@
 //         K-tiles, double-buffered in shared memory by cp.async; warp (y, bi, bj) accumulates
 //         the 32x32 super-block (bi, bj) of C_y in 16 mma tiles. Per-chunk partials are summed
 //         by gram2_reduce_kernel in a fixed order (deterministic).
-//  xt2:   Y = X T (n x k times k x nc, k, nc <= 96), persistent CTAs with T resident in shared
-//         memory. Plain form: 64-row tiles of X double-buffered, warp (slab, half) forms 16 rows x
-//         48 columns. Dual form (32-row tiles of X and W, 8-row warp slabs) also forms W T for the
-//         columns that need it and reduces
+//  xt2:   Y = X T (n x k times k x nc, k, nc <= 96) with W T beside it, persistent CTAs with T resident
+//         in shared memory, 32-row tiles of X and W, 8-row warp slabs (callback operators; plain products
+//         are in rc_xt.cu): W T is formed for the columns that need it, reducing
 //         ||(W T)_c - lam_c (X T)_c||^2 for c < res_count; with R32 it writes the residual block
 //         R = W T - (X T) diag(lam) in row-major FP32 (the source term of an FP32-storage
 //         correction filter; native real operators take R from rc_resid.cu instead).
@@ -23,28 +22,10 @@
 // B (4x8, col) b = B[q][g]; C (8x8) {c0, c1} = C[g][2q], C[g][2q+1].
 #include <algorithm>
 #include "rc_common.cuh"
+#include "rc_dmma.cuh"
 #include "rc_internal.h"
 
 namespace rcb {
-
-__device__ __forceinline__ void dmma(double& c0, double& c1, double a, double b) {
-    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
-                 : "+d"(c0), "+d"(c1)
-                 : "d"(a), "d"(b));
-}
-
-__device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
-
-// 16-byte (two rows) or 8-byte (one row) asynchronous copy global -> shared; bytes beyond
-// src_bytes are zero-filled (src_bytes = 0 reads nothing).
-__device__ __forceinline__ void cp_async16(void* dst, const void* src, int src_bytes) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(smem_u32(dst)), "l"(src), "r"(src_bytes));
-}
-__device__ __forceinline__ void cp_async8(void* dst, const void* src, int src_bytes) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(smem_u32(dst)), "l"(src), "r"(src_bytes));
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::); }
-__device__ __forceinline__ void cp_async_wait0() { asm volatile("cp.async.wait_group 0;\n" ::); }
 
 // Copy rows [r0, r0 + RT) of columns [0, ncols) of a column-major block into a shared tile laid
 // out column by column with `rp` doubles per column (rows past r_end read as zero).
@@ -488,14 +469,14 @@ __host__ __device__ inline int xm_kpt(int k) {
 }
 
 // Warps: 4 row slabs (8 rows each) x NH column halves (48 columns each).
-template <int NH, bool DUAL, bool V16>
+template <int NH, bool V16>
 __global__ void __launch_bounds__(128 * NH, 1)
 xt_mma_kernel(int64_t n, int k, int nc, const double* __restrict__ X, int64_t ldx, const double* __restrict__ Tm,
               int64_t ldt, double* __restrict__ Y, int64_t ldy, const double* __restrict__ W, int64_t ldw,
               const double* __restrict__ lam, int dual_cols, int res_count, double* __restrict__ rpart,
               float* __restrict__ R32, int64_t ldr) {
     constexpr int NT = 128 * NH;
-    constexpr int OPS = DUAL ? 2 : 1;
+    constexpr int OPS = 2;
     const int kpt = xm_kpt(k);
     const int k4 = (k + 3) / 4 * 4;
     extern __shared__ __align__(16) double xms[];
@@ -519,14 +500,14 @@ xt_mma_kernel(int64_t n, int k, int nc, const double* __restrict__ X, int64_t ld
         }
     }
     // mma tiles of this warp whose columns need W T (warp-uniform)
-    const int dtiles = DUAL ? max(0, min(XM_CT, (dual_cols - cbase + 7) / 8)) : 0;
+    const int dtiles = max(0, min(XM_CT, (dual_cols - cbase + 7) / 8));
     double lamc[XM_CT][2], rs[XM_CT][2];
 #pragma unroll
     for (int j = 0; j < XM_CT; ++j)
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
             const int c = cbase + j * 8 + 2 * q + h;
-            lamc[j][h] = (DUAL && c < dual_cols) ? lam[c] : 0.0;
+            lamc[j][h] = c < dual_cols ? lam[c] : 0.0;
             rs[j][h] = 0.0;
         }
     const int64_t ntiles = (n + XM_RT - 1) / XM_RT;
@@ -534,7 +515,7 @@ xt_mma_kernel(int64_t n, int k, int nc, const double* __restrict__ X, int64_t ld
         double* st = tiles + b * stage;
         const int64_t r0 = t * XM_RT;
         load_cols_async<XM_RT, V16>(st, XM_RP, X, ldx, k, r0, n, tid, NT);
-        if (DUAL) load_cols_async<XM_RT, V16>(st + k4 * XM_RP, XM_RP, W, ldw, k, r0, n, tid, NT);
+        load_cols_async<XM_RT, V16>(st + k4 * XM_RP, XM_RP, W, ldw, k, r0, n, tid, NT);
     };
     // two stages, one barrier per tile (as in gram_mma_kernel)
     int buf = 0;
@@ -561,7 +542,7 @@ xt_mma_kernel(int64_t n, int k, int nc, const double* __restrict__ X, int64_t ld
             for (int j = 0; j < XM_CT; ++j) b[j] = ts[j * 8 * kpt + k0];
 #pragma unroll
             for (int j = 0; j < XM_CT; ++j) dmma(acc[j][0], acc[j][1], a, b[j]);
-            if (DUAL && dtiles > 0) {
+            if (dtiles > 0) {
                 const double w = ws[k0 * XM_RP];
 #pragma unroll
                 for (int j = 0; j < XM_CT; ++j)
@@ -575,7 +556,7 @@ xt_mma_kernel(int64_t n, int k, int nc, const double* __restrict__ X, int64_t ld
                 const int c = cbase + j * 8 + 2 * q;
                 if (c < nc) Y[r + (int64_t)c * ldy] = acc[j][0];
                 if (c + 1 < nc) Y[r + (int64_t)(c + 1) * ldy] = acc[j][1];
-                if (DUAL && j < dtiles) {
+                if (j < dtiles) {
                     const double d0 = acc2[j][0] - lamc[j][0] * acc[j][0];
                     const double d1 = acc2[j][1] - lamc[j][1] * acc[j][1];
                     if (c < res_count) rs[j][0] = fma(d0, d0, rs[j][0]);
@@ -592,7 +573,7 @@ xt_mma_kernel(int64_t n, int k, int nc, const double* __restrict__ X, int64_t ld
         }
         buf ^= 1;
     }
-    if (DUAL && res_count > 0) {
+    if (res_count > 0) {
         __syncthreads();  // the last tile's reads are done before its stage is reused below
         // per column: sum over g (lanes with the same q), then over the four row slabs in order
         double* red = tiles;  // [4][NH*48]; the tiles are no longer read
@@ -616,104 +597,6 @@ xt_mma_kernel(int64_t n, int k, int nc, const double* __restrict__ X, int64_t ld
     }
 }
 
-// Plain product Y = X T (no dual): 64-row tiles, warp (slab, half) forms 16 rows x 48 columns
-// (two mma row tiles share each B fragment: 8 shared-memory reads per 12 mma).
-constexpr int XP_RT = 64;
-constexpr int XP_RP = XP_RT + 4;  // = 4 mod 16
-
-// X row-major (RM): the 64-row tiles are held row by row with kpt doubles per row (= 4 mod 16),
-// element (row r, column kk) at r * RS + kk * CS in both layouts.
-template <int NH, bool V16, bool RM = false>
-__global__ void __launch_bounds__(128 * NH, 1)
-xt_mma_plain_kernel(int64_t n, int k, int nc, const double* __restrict__ X, int64_t ldx,
-                    const double* __restrict__ Tm, int64_t ldt, double* __restrict__ Y, int64_t ldy,
-                    double* __restrict__ Yrm, int64_t ldyr) {
-    constexpr int NT = 128 * NH;
-    const int kpt = xm_kpt(k);
-    const int k4 = (k + 3) / 4 * 4;
-    extern __shared__ __align__(16) double xps[];
-    double* Ts = xps;                            // [NH*48][kpt]
-    double* tiles = Ts + (size_t)NH * 48 * kpt;  // [2][k4][XP_RP], or [2][XP_RT][kpt] when RM
-    const int stage = RM ? XP_RT * kpt : k4 * XP_RP;
-    const int CS = RM ? 1 : XP_RP, RS = RM ? kpt : 1;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int g = lane >> 2, q = lane & 3;
-    const int slab = warp & 3, half = warp >> 2;
-    const int cbase = half * 48;
-    for (int e = tid; e < NH * 48 * kpt; e += NT) {
-        const int c = e / kpt, kk = e - c * kpt;
-        Ts[e] = (c < nc && kk < k) ? Tm[kk + (int64_t)c * ldt] : 0.0;
-    }
-    if constexpr (RM) {  // padding columns k..k4 of every row of both stages
-        const int w = k4 - k;
-        for (int e = tid; e < 2 * XP_RT * w; e += NT) {
-            const int row = e / w;  // stage-major: row in [0, 2 * XP_RT)
-            tiles[row * kpt + k + (e - row * w)] = 0.0;
-        }
-    } else {
-        const int per = (k4 - k) * XP_RP;
-        for (int e = tid; e < 2 * per; e += NT) {
-            const int st = e / per, f = e - st * per;
-            tiles[st * stage + k * XP_RP + f] = 0.0;
-        }
-    }
-    const RowCopyMap rcm(k, tid, NT);
-    auto load = [&](double* dst, int64_t r0) {
-        if constexpr (RM) load_rows_async<XP_RT>(dst, kpt, X, ldx, k, r0, n, rcm);
-        else load_cols_async<XP_RT, V16>(dst, XP_RP, X, ldx, k, r0, n, tid, NT);
-    };
-    const int64_t ntiles = (n + XP_RT - 1) / XP_RT;
-    int buf = 0;
-    int64_t t = blockIdx.x;
-    if (t < ntiles) load(tiles, t * XP_RT);
-    cp_async_commit();
-    for (; t < ntiles; t += gridDim.x) {
-        cp_async_wait0();
-        __syncthreads();
-        const int64_t tn = t + gridDim.x;
-        if (tn < ntiles) load(tiles + (buf ^ 1) * stage, tn * XP_RT);
-        cp_async_commit();
-        const double* xs = tiles + buf * stage + (slab * 16 + g) * RS + q * CS;
-        const double* ts = Ts + (cbase + g) * kpt + q;
-        double acc[2][XM_CT][2];
-#pragma unroll
-        for (int m = 0; m < 2; ++m)
-#pragma unroll
-            for (int j = 0; j < XM_CT; ++j) acc[m][j][0] = acc[m][j][1] = 0.0;
-#pragma unroll 2
-        for (int k0 = 0; k0 < k4; k0 += 4) {
-            const double a0 = xs[k0 * CS], a1 = xs[k0 * CS + 8 * RS];
-            double b[XM_CT];
-#pragma unroll
-            for (int j = 0; j < XM_CT; ++j) b[j] = ts[j * 8 * kpt + k0];
-#pragma unroll
-            for (int j = 0; j < XM_CT; ++j) {
-                dmma(acc[0][j][0], acc[0][j][1], a0, b[j]);
-                dmma(acc[1][j][0], acc[1][j][1], a1, b[j]);
-            }
-        }
-#pragma unroll
-        for (int m = 0; m < 2; ++m) {
-            const int64_t r = t * XP_RT + slab * 16 + m * 8 + g;
-            if (r < n) {
-#pragma unroll
-                for (int j = 0; j < XM_CT; ++j) {
-                    const int c = cbase + j * 8 + 2 * q;
-                    if (c < nc) Y[r + (int64_t)c * ldy] = acc[m][j][0];
-                    if (c + 1 < nc) Y[r + (int64_t)(c + 1) * ldy] = acc[m][j][1];
-                    if (Yrm) {  // row-major copy (even leading dimension: 16-byte pairs)
-                        if (c + 1 < nc)
-                            *reinterpret_cast<double2*>(Yrm + r * ldyr + c) = make_double2(acc[m][j][0], acc[m][j][1]);
-                        else if (c < nc)
-                            Yrm[r * ldyr + c] = acc[m][j][0];
-                    }
-                }
-            }
-        }
-        buf ^= 1;
-    }
-}
-
 __global__ void resid2_reduce_kernel(int64_t nblocks, int res_count, const double* __restrict__ rpart,
                                      double* __restrict__ res) {
     const int c = blockIdx.x;
@@ -728,16 +611,16 @@ bool xt2_supported(int dtype, int64_t k, int64_t nc) {
     return dtype == RC_REAL64 && k >= 1 && k <= 96 && nc >= 1 && nc <= 96;
 }
 
-template <int NH, bool DUAL, bool V16>
+template <int NH, bool V16>
 static rc_status xt_mma_launch(rc_ctx* ctx, unsigned grid, int64_t n, int64_t k, int64_t nc, const double* X,
                                int64_t ldx, const double* T, int64_t ldt, double* Y, int64_t ldy, const double* W,
                                int64_t ldw, const double* lam, int64_t dual_cols, int64_t res_count, double* rpart,
                                float* R32, int64_t ldr) {
     const int k4 = (int)((k + 3) / 4 * 4);
     const size_t smem =
-        ((size_t)NH * 48 * xm_kpt((int)k) + (size_t)2 * (DUAL ? 2 : 1) * k4 * XM_RP) * sizeof(double);
-    RC_CU(ctx, allow_max_smem(ctx, xt_mma_kernel<NH, DUAL, V16>));
-    xt_mma_kernel<NH, DUAL, V16><<<grid, 128 * NH, smem, ctx->stream>>>(
+        ((size_t)NH * 48 * xm_kpt((int)k) + (size_t)4 * k4 * XM_RP) * sizeof(double);
+    RC_CU(ctx, allow_max_smem(ctx, xt_mma_kernel<NH, V16>));
+    xt_mma_kernel<NH, V16><<<grid, 128 * NH, smem, ctx->stream>>>(
         n, (int)k, (int)nc, X, ldx, T, ldt, Y, ldy, W, ldw, lam, (int)dual_cols, (int)res_count, rpart, R32, ldr);
     return RC_OK;
 }
@@ -746,12 +629,8 @@ static rc_status xt_mma_launch(rc_ctx* ctx, unsigned grid, int64_t n, int64_t k,
 // and with R32 the residual block (all nc columns) in row-major FP32 with leading dimension ldr.
 rc_status xt2(rc_ctx* ctx, int64_t n, int64_t k, int64_t nc, const double* X, int64_t ldx, const double* T,
               int64_t ldt, double* Y, int64_t ldy, const double* W, int64_t ldw, const double* lam, int64_t res_count,
-              double* res, float* R32, int64_t ldr, double* Yrm, int64_t ldyr) {
+              double* res, float* R32, int64_t ldr) {
     const bool dual = W != nullptr && lam != nullptr && (res_count > 0 || R32 != nullptr);
-    if (!dual) {
-        res_count = 0;
-        R32 = nullptr;
-    }
     const int64_t dual_cols = dual ? (R32 ? nc : std::min(res_count, nc)) : 0;
     if (R32 && (ldr % 2 != 0 || (uintptr_t)R32 % 8 != 0))
         return rc_fail(ctx, RC_ERR_INVALID, "xt2: the residual block needs an even leading dimension");
@@ -766,35 +645,14 @@ rc_status xt2(rc_ctx* ctx, int64_t n, int64_t k, int64_t nc, const double* X, in
     }
     const bool v16 =
         ((uintptr_t)X % 16 == 0) && (ldx % 2 == 0) && (!dual || (((uintptr_t)W % 16 == 0) && ldw % 2 == 0));
-    if (Yrm && (dual || ldyr % 2 != 0 || (uintptr_t)Yrm % 16 != 0))
-        return rc_fail(ctx, RC_ERR_INVALID, "xt2: the row-major copy needs the plain product and an even leading dimension");
-    if (!dual) {
-        const int64_t pt = (n + XP_RT - 1) / XP_RT;
-        const unsigned pg = (unsigned)std::max<int64_t>(1, std::min<int64_t>(pt, ctx->sm_count));
-        const size_t psm = ((size_t)nh * 48 * xm_kpt((int)k) + (size_t)2 * ((k + 3) / 4 * 4) * XP_RP) * sizeof(double);
-#define RC_XP(NHV, VV)                                                                                            \
-    do {                                                                                                          \
-        RC_CU(ctx, allow_max_smem(ctx, xt_mma_plain_kernel<NHV, VV>));                                            \
-        xt_mma_plain_kernel<NHV, VV><<<pg, 128 * NHV, psm, ctx->stream>>>(n, (int)k, (int)nc, X, ldx, T, ldt, Y, ldy, \
-                                                                          Yrm, ldyr);                            \
-    } while (0)
-        if (nh == 1) {
-            if (v16) RC_XP(1, true); else RC_XP(1, false);
-        } else {
-            if (v16) RC_XP(2, true); else RC_XP(2, false);
-        }
-#undef RC_XP
-        ctx->launches++;
-        RC_CU(ctx, cudaGetLastError());
-        return RC_OK;
-    }
-#define RC_XM(NHV, DV)                                                                                            \
-    (v16 ? xt_mma_launch<NHV, DV, true>(ctx, grid, n, k, nc, X, ldx, T, ldt, Y, ldy, W, ldw, lam, dual_cols,      \
-                                        res_count, rpart, R32, ldr)                                               \
-         : xt_mma_launch<NHV, DV, false>(ctx, grid, n, k, nc, X, ldx, T, ldt, Y, ldy, W, ldw, lam, dual_cols,     \
-                                         res_count, rpart, R32, ldr))
+    if (!dual) return rc_fail(ctx, RC_ERR_INVALID, "xt2: the second block is required");
+#define RC_XM(NHV)                                                                                                \
+    (v16 ? xt_mma_launch<NHV, true>(ctx, grid, n, k, nc, X, ldx, T, ldt, Y, ldy, W, ldw, lam, dual_cols, res_count, \
+                                    rpart, R32, ldr)                                                              \
+         : xt_mma_launch<NHV, false>(ctx, grid, n, k, nc, X, ldx, T, ldt, Y, ldy, W, ldw, lam, dual_cols, res_count, \
+                                     rpart, R32, ldr))
     rc_status st;
-    st = nh == 1 ? RC_XM(1, true) : RC_XM(2, true);
+    st = nh == 1 ? RC_XM(1) : RC_XM(2);
 #undef RC_XM
     RC_TRY(st);
     ctx->launches++;
@@ -804,34 +662,6 @@ rc_status xt2(rc_ctx* ctx, int64_t n, int64_t k, int64_t nc, const double* X, in
         ctx->launches++;
         RC_CU(ctx, cudaGetLastError());
     }
-    return RC_OK;
-}
-
-// Y = X T for a row-major X (leading dimension ldx, even, >= k, rows 16-byte aligned): Y column-major
-// (ldy) and, when Yrm is given, a row-major copy (ldyr, even).
-rc_status xt2_rm(rc_ctx* ctx, int64_t n, int64_t k, int64_t nc, const double* X, int64_t ldx, const double* T,
-                 int64_t ldt, double* Y, int64_t ldy, double* Yrm, int64_t ldyr) {
-    if (!xt2_supported(RC_REAL64, k, nc)) return rc_fail(ctx, RC_ERR_UNSUPPORTED, "xt2_rm: k, nc <= 96 only");
-    if ((uintptr_t)X % 16 != 0 || ldx % 2 != 0 || ldx < k)
-        return rc_fail(ctx, RC_ERR_INVALID, "xt2_rm: row-major X needs an even leading dimension >= k, 16-byte aligned");
-    if (Yrm && (ldyr % 2 != 0 || (uintptr_t)Yrm % 16 != 0))
-        return rc_fail(ctx, RC_ERR_INVALID, "xt2_rm: the row-major copy needs an even leading dimension");
-    const int nh = nc <= 48 ? 1 : 2;
-    const int64_t pt = (n + XP_RT - 1) / XP_RT;
-    const unsigned pg = (unsigned)std::max<int64_t>(1, std::min<int64_t>(pt, ctx->sm_count));
-    const int kpt = xm_kpt((int)k);
-    const size_t psm = ((size_t)nh * 48 * kpt + (size_t)2 * XP_RT * kpt) * sizeof(double);
-    if (nh == 1) {
-        RC_CU(ctx, allow_max_smem(ctx, xt_mma_plain_kernel<1, true, true>));
-        xt_mma_plain_kernel<1, true, true><<<pg, 128, psm, ctx->stream>>>(n, (int)k, (int)nc, X, ldx, T, ldt, Y,
-                                                                          ldy, Yrm, ldyr);
-    } else {
-        RC_CU(ctx, allow_max_smem(ctx, xt_mma_plain_kernel<2, true, true>));
-        xt_mma_plain_kernel<2, true, true><<<pg, 256, psm, ctx->stream>>>(n, (int)k, (int)nc, X, ldx, T, ldt, Y,
-                                                                          ldy, Yrm, ldyr);
-    }
-    ctx->launches++;
-    RC_CU(ctx, cudaGetLastError());
     return RC_OK;
 }
 

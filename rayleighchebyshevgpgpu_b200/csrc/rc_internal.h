@@ -115,7 +115,7 @@ struct rc_ctx {
 
 enum Slot {
     S_V = 0, S_W, S_T1, S_T2, S_FOUND, S_PART, S_SMALL, S_LANCZOS, S_RPART, S_IO, S_CB, S_EIG, S_FA, S_FB,
-    S_R32, S_CORR, S_YRM, S_BATCH, S_VFRM, S_WRM, S_PAIR, S_COUNT
+    S_R32, S_CORR, S_YRM, S_BATCH, S_VFRM, S_WRM, S_PAIR, S_XTP, S_COUNT
 };
 
 struct rc_op {
@@ -271,7 +271,8 @@ void step_flush(rc_ctx* ctx);
 // (requires m == nc and a Hermitian result). part: scratch for per-chunk partial sums.
 rc_status gram(rc_ctx* ctx, int dtype, int64_t n, int64_t m, int64_t nc, const void* X, int64_t ldx,
                const void* Y, int64_t ldy, void* C, bool upper);
-// Y (n x nc) = beta*Y + alpha * X (n x k) * T (k x nc, ld ldt). Y must not alias X.
+// Y (n x nc) = beta*Y + alpha * X (n x k) * T (k x nc, ld ldt). Y must not alias X, except as xt_dmma allows
+// it for plain products.
 // Optional dual: X2 * T (stored in Y2 unless Y2 is null) and residual norms
 // ||(X2 T)_c - lam_c Y_c|| for c < res_count.
 struct XtArgs {
@@ -288,14 +289,14 @@ struct XtArgs {
     // optional: the residual block X2 T - Y diag(lam) (all nc columns) in row-major FP32 with
     // leading dimension ldr (real blocks with k, nc <= 96 only)
     float* R32 = nullptr; int64_t ldr = 0;
-    // optional: a row-major FP64 copy of Y (plain products, real blocks with k, nc <= 96)
+    // optional: a row-major FP64 copy of Y (plain products, real blocks)
     double* Yrm = nullptr; int64_t ldyr = 0;
 };
 rc_status xt(rc_ctx* ctx, int dtype, const XtArgs& a);
 
 // FP64 real fast paths (s <= 96), rc_gemm.cu. gram2: C0 = X^T Y0 (and C1 = X^T Y1 when Y1),
-// symmetric results. xt2: Y = X T, plus residual norms of W T against lam when W is given, and
-// the residual block W T - Y diag(lam) in row-major FP32 when R32 is given.
+// symmetric results. xt2: Y = X T with the residual norms of W T against lam, and the residual block
+// W T - Y diag(lam) in row-major FP32 when R32 is given.
 bool gram2_supported(int dtype, int64_t m);
 // Complex Hermitian Gram C = X^H Y (m x m, m <= 192, column-major, upper formed and mirrored) on the
 // FP64 tensor pipe.
@@ -305,12 +306,20 @@ rc_status gram_c(rc_ctx* ctx, int64_t n, int64_t m, const double2* X, int64_t ld
 rc_status gram2(rc_ctx* ctx, int64_t n, int64_t m, const double* X, int64_t ldx, const double* Y0, int64_t ldy0,
                 double* C0, const double* Y1, int64_t ldy1, double* C1, bool rm = false);
 bool xt2_supported(int dtype, int64_t k, int64_t nc);
-// Y = X T with X row-major (leading dimension ldx): Y column-major and, with Yrm, row-major.
-rc_status xt2_rm(rc_ctx* ctx, int64_t n, int64_t k, int64_t nc, const double* X, int64_t ldx, const double* T,
-                 int64_t ldt, double* Y, int64_t ldy, double* Yrm, int64_t ldyr);
 rc_status xt2(rc_ctx* ctx, int64_t n, int64_t k, int64_t nc, const double* X, int64_t ldx, const double* T,
               int64_t ldt, double* Y, int64_t ldy, const double* W, int64_t ldw, const double* lam, int64_t res_count,
-              double* res, float* R32 = nullptr, int64_t ldr = 0, double* Yrm = nullptr, int64_t ldyr = 0);
+              double* res, float* R32 = nullptr, int64_t ldr = 0);
+// Y = alpha X T + beta Y on the FP64 tensor pipe (rc_xt.cu): any dtype and width, X column-major or
+// (real, x_rm) row-major, and with Yrm (real) a row-major copy of Y. Y may be X when T is square and
+// xt_dmma_in_place(nc).
+bool xt_dmma_in_place(int64_t nc);
+rc_status xt_dmma(rc_ctx* ctx, int dtype, int64_t n, int64_t k, int64_t nc, const void* X, int64_t ldx, bool x_rm,
+                  const void* T, int64_t ldt, void* Y, int64_t ldy, double alpha = 1.0, double beta = 0.0,
+                  double* Yrm = nullptr, int64_t ldyr = 0);
+
+// res[c] = ||W_c - lam_c V_c|| for c < res_count (device), column-major blocks (rc_resid.cu).
+rc_status resid_norms(rc_ctx* ctx, int dtype, int64_t n, int64_t res_count, const void* V, int64_t ldv, const void* W,
+                      int64_t ldw, const double* lam, double* res);
 
 // Residual block of Ritz vectors on native operators (rc_resid.cu; real, or complex CSR and 5/7-point
 // stencils; s <= kCorrMaxCols): R = A Y - Y diag(lam) from the row-major FP64 (c128) copy Yrm of Y

@@ -225,6 +225,49 @@ __global__ void resid_norm_reduce_kernel(int64_t nparts, int res_count, const do
     if (threadIdx.x == 0) res[c] = sqrt(v);
 }
 
+// Residual norms of column-major blocks: chunk blockIdx.x of column blockIdx.y. One read of both blocks
+// (their HBM bandwidth is the bound); part[chunk * res_count + c], summed by resid_norm_reduce_kernel.
+template <class T>
+__global__ void __launch_bounds__(256)
+resid_norms_kernel(int64_t n, int res_count, int64_t rows, const T* __restrict__ V, int64_t ldv,
+                   const T* __restrict__ W, int64_t ldw, const double* __restrict__ lam, double* __restrict__ part) {
+    __shared__ double sc[32];
+    const int c = blockIdx.y;
+    const double lm = lam[c];
+    const int64_t r0 = (int64_t)blockIdx.x * rows, r1 = min(n, r0 + rows);
+    const T* v = V + (int64_t)c * ldv;
+    const T* w = W + (int64_t)c * ldw;
+    double s = 0.0;
+#pragma unroll 4
+    for (int64_t i = r0 + threadIdx.x; i < r1; i += 256) s += s_abs2(resid_sub(lm, __ldcs(v + i), __ldcs(w + i)));
+    s = block_sum(s, sc);
+    if (threadIdx.x == 0) part[(int64_t)blockIdx.x * res_count + c] = s;
+}
+
+rc_status resid_norms(rc_ctx* ctx, int dtype, int64_t n, int64_t res_count, const void* V, int64_t ldv, const void* W,
+                      int64_t ldw, const double* lam, double* res) {
+    if (res_count < 1) return RC_OK;
+    if (res_count > 65535) return rc_fail(ctx, RC_ERR_UNSUPPORTED, "residual norms: too many columns");
+    const int64_t rows = 8192;
+    const int64_t chunks = (n + rows - 1) / rows;
+    void* part = nullptr;
+    RC_TRY(rc_slot(ctx, S_RPART, (size_t)chunks * res_count * sizeof(double), &part));
+    const dim3 grid((unsigned)chunks, (unsigned)res_count);
+    if (dtype == RC_COMPLEX128)
+        resid_norms_kernel<double2><<<grid, 256, 0, ctx->stream>>>(n, (int)res_count, rows, (const double2*)V, ldv,
+                                                                   (const double2*)W, ldw, lam, (double*)part);
+    else
+        resid_norms_kernel<double><<<grid, 256, 0, ctx->stream>>>(n, (int)res_count, rows, (const double*)V, ldv,
+                                                                  (const double*)W, ldw, lam, (double*)part);
+    ctx->launches++;
+    RC_CU(ctx, cudaGetLastError());
+    resid_norm_reduce_kernel<<<(unsigned)res_count, 256, 0, ctx->stream>>>(chunks, (int)res_count, (const double*)part,
+                                                                           res);
+    ctx->launches++;
+    RC_CU(ctx, cudaGetLastError());
+    return RC_OK;
+}
+
 bool resid_supported(const rc_op* op, int64_t s) {
     if (s < 1 || s > kCorrMaxCols || op->kind == 2) return false;
     if (op->dtype == RC_REAL64) return op->kind == 0 || op->skind == 5 || op->skind == 7 || op->skind == 27;

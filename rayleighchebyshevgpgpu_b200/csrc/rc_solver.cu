@@ -234,7 +234,7 @@ rc_status Solver::ortho(int64_t s) {
 // Ritz vectors Y = X Q (a.Y) and the residuals of their first res_count columns (dres_), plus
 // the correction filter's residual block when R32 is given. Native operators (real, or complex CSR
 // and 5/7-point stencils) with s <= kCorrMaxCols: Y by the GEMM and a row-major FP64 (c128) copy of
-// it (written by the real GEMM itself for s <= 96, else by a layout change), then
+// it (written by the real GEMM itself, else by a layout change), then
 // R = A Y - Y diag(lam) in one pass over that copy (rc_resid.cu): a sparse product costs less than
 // the second dense product W Q. Otherwise (callback operators, wider blocks): the dual GEMM (A X) Q
 // with the residual norms reduced on the fly.
@@ -248,7 +248,7 @@ rc_status Solver::ritz_and_residuals(XtArgs a, int64_t s, int64_t res_count, voi
         a.Y2 = nullptr;
         a.lam = nullptr;
         a.res_count = 0;
-        if (dtype_ == RC_REAL64 && xt2_supported(dtype_, a.k, a.nc)) {
+        if (dtype_ == RC_REAL64) {
             a.Yrm = (double*)yrm;
             a.ldyr = ldrm;
             RC_TRY(xt(ctx_, dtype_, a));
@@ -356,8 +356,7 @@ rc_status Solver::rr_fused(int64_t s, int64_t res_count, bool* ok, void* R32) {
         // Ritz vectors V_f Q, column-major into T1_ and row-major beside them, then the residuals
         void* yrm = nullptr;
         RC_TRY(rc_slot(ctx_, S_YRM, (size_t)n_ * ldrm * sizeof(double), &yrm));
-        RC_TRY(xt2_rm(ctx_, n_, s, s, (const double*)vf, ldrm, (const double*)Q_, s, (double*)T1_, n_, (double*)yrm,
-                      ldrm));
+        RC_TRY(xt_dmma(ctx_, dtype_, n_, s, s, vf, ldrm, true, Q_, s, T1_, n_, 1.0, 0.0, (double*)yrm, ldrm));
         RC_TRY(resid_block(ctx_, op_, yrm, ldrm, s, dlam_, res_count, dres_, R32,
                            R32 ? corr_leading_dim(dtype_, s) : 0));
         rWritten_ = R32 != nullptr;
