@@ -575,6 +575,32 @@ __device__ __forceinline__ void jac_qrot(T& qp, T& qq, double cj, double sj, T u
     qp = np;
 }
 
+// The power of two 2^sh by which a matrix is scaled down (exactly) so that its entries are at most 1 and their
+// squares neither overflow nor underflow; the same in every CTA.
+template <class T>
+__device__ __forceinline__ int jac_scale(const T* __restrict__ A, int s, double* red) {
+    double mx = 0.0;
+    for (int e = threadIdx.x; e < s * s; e += blockDim.x) {
+        const T v = A[e];
+        mx = fmax(mx, fmax(fabs(s_real(v)), fabs(s_imag(v))));
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+    __syncthreads();
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = mx;
+    __syncthreads();
+    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) mx = fmax(mx, red[w]);
+    __syncthreads();
+    int sh = 0;
+    if (mx > 0.0 && isfinite(mx)) frexp(mx, &sh);
+    return sh;
+}
+template <class T>
+__device__ __forceinline__ T jac_scaled(T v, int sh) {
+    if (sh == 0) return v;
+    return s_rscale(ldexp(1.0, -sh - (-sh / 2)), s_rscale(ldexp(1.0, -sh / 2), v));
+}
+
 // Threads of the one-CTA Jacobi (a multiple of 32, at most 1024).
 #ifndef RC_JACOBI_THREADS
 #define RC_JACOBI_THREADS 1024
@@ -583,7 +609,7 @@ __device__ __forceinline__ void jac_qrot(T& qp, T& qq, double cj, double sj, T u
 template <class T>
 __global__ void __launch_bounds__(1024)
 jacobi_kernel(int s, const T* __restrict__ Ain, T* __restrict__ Qout, double* __restrict__ evals, int* info,
-              T* work, int use_smem, int max_sweeps) {
+              T* work, int max_sweeps) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int sp = s + (s & 1);  // even number of indices (one zero dummy row/column when s is odd)
     const int npair = sp / 2;
@@ -593,24 +619,19 @@ jacobi_kernel(int s, const T* __restrict__ Ain, T* __restrict__ Qout, double* __
     T* ru = (T*)(rsn + npair);
     int* pp = (int*)(ru + npair);
     int* qq = pp + npair;
-    T* A;
-    T* Q;
-    if (use_smem) {
-        A = (T*)((char*)smem_raw + (((size_t)npair * (16 + sizeof(T) + 8) + 15) / 16) * 16);
-    } else {
-        A = work;
-    }
-    Q = A + (size_t)sp * ld;
+    T* A = work;
+    T* Q = A + (size_t)sp * ld;
     const int tid = threadIdx.x, nt = blockDim.x;
-    for (int e = tid; e < sp * sp; e += nt) {
-        const int i = e % sp, j = e / sp;
-        A[i + j * ld] = (i < s && j < s) ? Ain[i + (int64_t)j * s] : s_zero(T());
-        Q[i + j * ld] = s_from<T>(i == j ? 1.0 : 0.0, 0.0);
-    }
     __shared__ double s_fro;
     __shared__ int s_rot;
     __shared__ unsigned long long s_maxsn;  // largest |sin| of the sweep's rotations (bits of a positive double)
     __shared__ double red[32];
+    const int sh = jac_scale(Ain, s, red);
+    for (int e = tid; e < sp * sp; e += nt) {
+        const int i = e % sp, j = e / sp;
+        A[i + j * ld] = (i < s && j < s) ? jac_scaled(Ain[i + (int64_t)j * s], sh) : s_zero(T());
+        Q[i + j * ld] = s_from<T>(i == j ? 1.0 : 0.0, 0.0);
+    }
     __syncthreads();
     double f = 0.0;
     for (int e = tid; e < sp * sp; e += nt) f += s_abs2(A[(e % sp) + (e / sp) * ld]);
@@ -739,7 +760,7 @@ jacobi_kernel(int s, const T* __restrict__ Ain, T* __restrict__ Qout, double* __
             const double lj = s_real(A[j + j * ld]);
             if (lj < li || (lj == li && j < i)) ++rank;
         }
-        evals[rank] = li;
+        evals[rank] = ldexp(li, sh);
         for (int row = 0; row < s; ++row) Qout[row + (int64_t)rank * s] = Q[row + i * ld];
     }
     if (tid == 0 && info) info[0] = sweep;
@@ -833,18 +854,19 @@ jacobi_grid_kernel(int s, const T* __restrict__ Ain, T* __restrict__ Qout, doubl
     const int G = gridDim.x, b = blockIdx.x;
     unsigned gen = 0;
     bool ok = true;
+    const int sh = jac_scale(Ain, s, red);
     // working copies: CTA b initialises its share of the entries
     {
         const int64_t tot = (int64_t)sp * sp;
         for (int64_t e = (int64_t)b * nt + tid; e < tot; e += (int64_t)G * nt) {
             const int i = (int)(e % sp), j = (int)(e / sp);
-            __stcg(Abuf[0] + i + (int64_t)j * ld, (i < s && j < s) ? Ain[i + (int64_t)j * s] : s_zero(T()));
+            __stcg(Abuf[0] + i + (int64_t)j * ld, (i < s && j < s) ? jac_scaled(Ain[i + (int64_t)j * s], sh) : s_zero(T()));
             __stcg(Q + i + (int64_t)j * ld, s_from<T>(i == j ? 1.0 : 0.0, 0.0));
         }
     }
     // the Frobenius norm of the input, in the same order in every CTA
     double f = 0.0;
-    for (int e = tid; e < s * s; e += nt) f += s_abs2(Ain[e]);
+    for (int e = tid; e < s * s; e += nt) f += s_abs2(jac_scaled(Ain[e], sh));
     f = block_sum(f, red);
     const double abs_tol = 1e-17 * sqrt(f);
     const double rel_tol = 1e-15;
@@ -1003,20 +1025,18 @@ jacobi_grid_kernel(int s, const T* __restrict__ Ain, T* __restrict__ Qout, doubl
             if (lj < li || (lj == li && j < i)) ++rank;
         }
         rank = (int)block_sum((double)rank, red);
-        if (tid == 0) evals[rank] = li;
+        if (tid == 0) evals[rank] = ldexp(li, sh);
         for (int row = tid; row < s; row += nt) Qout[row + (int64_t)rank * s] = __ldcg(Q + row + (int64_t)i * ld);
     }
     if (b == 0 && tid == 0 && info) info[0] = sweep;
 }
 
 size_t small_eigh_work_bytes(rc_ctx* ctx, int dtype, int64_t s) {
+    if (jacobi_cluster_ctas(ctx, dtype, s) > 0) return 0;
     const size_t esz = dtype == RC_COMPLEX128 ? 16 : 8;
     const int64_t sp = s + (s & 1);
-    const int64_t npair = sp / 2;
-    const size_t head = (((size_t)npair * (16 + esz + 8) + 15) / 16) * 16;
-    const size_t mats = 2 * (size_t)sp * (sp + 1) * esz;
-    // in global memory the grid form keeps A twice (3 matrices); the one-CTA kernel uses 2 of them
-    return head + mats <= (size_t)ctx->smem_optin - 2048 ? 0 : 3 * (size_t)sp * (sp + 1) * esz;
+    // the grid form keeps A twice (3 matrices); the one-CTA kernel uses 2 of them
+    return 3 * (size_t)sp * (sp + 1) * esz;
 }
 
 rc_status small_eigh(rc_ctx* ctx, int dtype, int64_t s, void* A, void* Q, double* evals, int* info) {
@@ -1031,38 +1051,32 @@ rc_status small_eigh_work(rc_ctx* ctx, int dtype, int64_t s, void* A, void* Q, d
     const int64_t sp = s + (s & 1);
     const int64_t npair = sp / 2;
     const size_t head = (((size_t)npair * (16 + esz + 8) + 15) / 16) * 16;
-    const size_t mats = 2 * (size_t)sp * (sp + 1) * esz;
-    const bool fit = head + mats <= (size_t)ctx->smem_optin - 2048;
-    const size_t dyn = fit ? head + mats : head;
-    if (!fit && !work) return rc_fail(ctx, RC_ERR_INVALID, "small_eigh: work memory required");
     const int sweeps = 60;
+    const int cluster = jacobi_cluster_ctas(ctx, dtype, s);
+    if (cluster > 0) return jacobi_cluster(ctx, dtype, s, cluster, A, Q, evals, info, sweeps);
+    if (!work) return rc_fail(ctx, RC_ERR_INVALID, "small_eigh: work memory required");
     // working copies in global memory: the grid form over up to 32 CTAs (RCB200_JACOBI_CTAS; 1 keeps
     // the one-CTA kernel), launched cooperatively, with its barrier words in info[1..3]
     const int ctas = std::max(1, std::min(ctx->jacobi_ctas > 0 ? ctx->jacobi_ctas : 32, ctx->sm_count));
-    if (!fit && ctas > 1 && info) {
+    if (ctas > 1 && info) {
         RC_CU(ctx, cudaMemsetAsync(info + 1, 0, 3 * sizeof(int), ctx->stream));
         int si = (int)s;
         int sw = sweeps;
         void* args[] = {&si, &A, &Q, &evals, &info, &work, &sw};
         const void* kern = dtype == RC_COMPLEX128 ? (const void*)jacobi_grid_kernel<double2>
                                                   : (const void*)jacobi_grid_kernel<double>;
-        RC_CU(ctx, cudaLaunchCooperativeKernel(kern, dim3((unsigned)ctas), dim3(kJacGridThreads), args, dyn,
+        RC_CU(ctx, cudaLaunchCooperativeKernel(kern, dim3((unsigned)ctas), dim3(kJacGridThreads), args, head,
                                                ctx->stream));
         ctx->launches++;
         return RC_OK;
     }
     const int nthr = ctx->jacobi_threads > 0 ? ctx->jacobi_threads : RC_JACOBI_THREADS;
-    if (dtype == RC_COMPLEX128) {
-        if (dyn > 48 * 1024)
-            RC_CU(ctx, allow_max_smem(ctx, jacobi_kernel<double2>));
-        jacobi_kernel<double2><<<1, nthr, dyn, ctx->stream>>>((int)s, (const double2*)A, (double2*)Q, evals, info,
-                                                              (double2*)work, fit ? 1 : 0, sweeps);
-    } else {
-        if (dyn > 48 * 1024)
-            RC_CU(ctx, allow_max_smem(ctx, jacobi_kernel<double>));
-        jacobi_kernel<double><<<1, nthr, dyn, ctx->stream>>>((int)s, (const double*)A, (double*)Q, evals, info,
-                                                             (double*)work, fit ? 1 : 0, sweeps);
-    }
+    if (dtype == RC_COMPLEX128)
+        jacobi_kernel<double2><<<1, nthr, head, ctx->stream>>>((int)s, (const double2*)A, (double2*)Q, evals, info,
+                                                               (double2*)work, sweeps);
+    else
+        jacobi_kernel<double><<<1, nthr, head, ctx->stream>>>((int)s, (const double*)A, (double*)Q, evals, info,
+                                                              (double*)work, sweeps);
     ctx->launches++;
     RC_CU(ctx, cudaGetLastError());
     return RC_OK;

@@ -48,6 +48,9 @@ struct rc_ctx {
     // pinned host staging for small read-backs
     double* host_small = nullptr;
     size_t host_small_bytes = 0;
+    // and for rc_small_eigh's matrices (its own: an operator callback may call it during a solve)
+    void* host_eigh = nullptr;
+    size_t host_eigh_bytes = 0;
     int sm_count = 148;
     size_t smem_optin = 232448;
     // operators created on this context; rc_ctx_destroy releases the ones still alive
@@ -76,12 +79,15 @@ struct rc_ctx {
     // stencil-structured operators: 1, or 0 (default: the per-row gather kernels, measured faster
     // on the 128^3 workloads), from RCB200_STAGED.
     int staged = 0;
-    // CTAs of the Jacobi eigensolve when its working copies live in global memory (0 = 32; 1 = the
-    // one-CTA kernel), from RCB200_JACOBI_CTAS.
+    // CTAs of the Jacobi eigensolve, from RCB200_JACOBI_CTAS (0: by size): at most 8 for the cluster kernel, which
+    // takes more where fewer cannot hold the matrix only when 0; otherwise of the kernels with the working copies in
+    // global memory (0 = 32; 1 = one CTA).
     int jacobi_ctas = 0;
-    // Threads of the one-CTA Jacobi kernel (0 = 1024), from RCB200_JACOBI_THREADS; jacobi_sweeps is
+    // Threads per CTA of the Jacobi kernels in shared memory and of one CTA (0: by size), from RCB200_JACOBI_THREADS; jacobi_sweeps is
     // the number of sweeps the last rc_small_eigh call ran.
     int jacobi_threads = 0;
+    // whether 16-CTA clusters run here, real and complex kernel (-1: not asked yet)
+    int jacobi16_r = -1, jacobi16_c = -1;
     // Complex Hermitian Gram products (m <= 192) on the FP64 tensor pipe (gram_c): 1 (default), or 0
     // for the FP64 SIMT kernel, from RCB200_GRAM_C.
     int gram_c = 1;
@@ -341,6 +347,10 @@ rc_status small_eigh(rc_ctx* ctx, int dtype, int64_t s, void* A, void* Q, double
 // copies fit in shared memory; 256-byte aligned).
 size_t small_eigh_work_bytes(rc_ctx* ctx, int dtype, int64_t s);
 rc_status small_eigh_work(rc_ctx* ctx, int dtype, int64_t s, void* A, void* Q, double* evals, int* info, void* work);
+// The Jacobi in the shared memory of one cluster (rc_jacobi.cu): CTAs it takes (0: too large), and its launch.
+int jacobi_cluster_ctas(rc_ctx* ctx, int dtype, int64_t s);
+rc_status jacobi_cluster(rc_ctx* ctx, int dtype, int64_t s, int ctas, const void* A, void* Q, double* evals, int* info,
+                         int max_sweeps);
 // C = op(A) B for s x s matrices (op = conjugate transpose when transA), and C <- (C + C^H)/2.
 rc_status small_gemm(rc_ctx* ctx, int dtype, int64_t s, const void* A, bool transA, const void* B, void* C);
 rc_status hermitize(rc_ctx* ctx, int dtype, int64_t s, void* C);
