@@ -1,6 +1,7 @@
 // rc_dmma.cuh -- FP64 tensor-pipe and cp.async primitives of the tall-skinny products
 // (rc_gemm.cu, rc_xt.cu).
 #pragma once
+#include <cuda.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -53,6 +54,14 @@ __device__ __forceinline__ void bulk_copy(uint32_t dst, const void* src, unsigne
                  "l"(src), "r"(bytes), "r"(bar)
                  : "memory");
 }
+// One tile of a 2-D tensor map, starting at (x, y): x a multiple of 16 bytes, dst of 128. What lies outside reads
+// as zero, and the whole tile's bytes are counted.
+__device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, int x, int y, uint32_t bar) {
+    asm volatile(
+        "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
+        ::"r"(dst), "l"(map), "r"(x), "r"(y), "r"(bar)
+        : "memory");
+}
 // Wait for the phase of the given parity. Bounded (each try suspends for a while by itself): false when the
 // limit ran out, which only a lost copy could cause.
 constexpr int kMbarTries = 1 << 22;
@@ -67,6 +76,30 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, unsigned parity) {
         if (ok) return true;
     }
     return false;
+}
+
+// A tensor map of doubles: `inner` consecutive ones in each of `outer` rows, `ld` apart (ld even, p 16-byte
+// aligned), tiles of box_inner x box_outer, not swizzled. False when the driver refuses it.
+inline bool tma_map_2d(CUtensorMap* map, const double* p, int64_t inner, int64_t outer, int64_t ld, int box_inner,
+                       int box_outer) {
+    typedef CUresult (*Fn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
+                           const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
+                           CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+    static Fn fn = [] {  // through the runtime: no link-time dependency on libcuda
+        void* f = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &f, cudaEnableDefault, &q) != cudaSuccess ||
+            q != cudaDriverEntryPointSuccess)
+            f = nullptr;
+        return (Fn)f;
+    }();
+    if (!fn) return false;
+    const cuuint64_t dims[2] = {(cuuint64_t)inner, (cuuint64_t)outer};
+    const cuuint64_t strides[1] = {(cuuint64_t)ld * sizeof(double)};
+    const cuuint32_t box[2] = {(cuuint32_t)box_inner, (cuuint32_t)box_outer}, es[2] = {1, 1};
+    return fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 2, const_cast<double*>(p), dims, strides, box, es,
+              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
 }  // namespace rcb

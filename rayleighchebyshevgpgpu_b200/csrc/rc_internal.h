@@ -300,17 +300,13 @@ struct XtArgs {
 };
 rc_status xt(rc_ctx* ctx, int dtype, const XtArgs& a);
 
-// FP64 real fast paths (s <= 96), rc_gemm.cu. gram2: C0 = X^T Y0 (and C1 = X^T Y1 when Y1),
-// symmetric results. xt2: Y = X T with the residual norms of W T against lam, and the residual block
-// W T - Y diag(lam) in row-major FP32 when R32 is given.
-bool gram2_supported(int dtype, int64_t m);
-// Complex Hermitian Gram C = X^H Y (m x m, m <= 192, column-major, upper formed and mirrored) on the
-// FP64 tensor pipe.
-bool gram_c_supported(int dtype, int64_t m);
-rc_status gram_c(rc_ctx* ctx, int64_t n, int64_t m, const double2* X, int64_t ldx, const double2* Y, int64_t ldy,
-                 double2* C);
-rc_status gram2(rc_ctx* ctx, int64_t n, int64_t m, const double* X, int64_t ldx, const double* Y0, int64_t ldy0,
-                double* C0, const double* Y1, int64_t ldy1, double* C1, bool rm = false);
+// C = X^H X (CX) and / or X^H W (CW), m x m, upper triangles formed and mirrored, on the FP64 tensor pipe
+// (rc_gram.cu): column-major, up to 192 columns (complex blocks 16-byte aligned), or row-major (rm: real, up to 96).
+bool gram_dmma_supported(int64_t m, bool rm);
+rc_status gram_dmma(rc_ctx* ctx, int dtype, int64_t n, int64_t m, const void* X, int64_t ldx, void* CX, const void* W,
+                    int64_t ldw, void* CW, bool rm);
+// The dual product for callback operators (rc_gemm.cu; real, k, nc <= 96): Y = X T with the residual norms of
+// W T against lam, and the residual block W T - Y diag(lam) in row-major FP32 when R32 is given.
 bool xt2_supported(int dtype, int64_t k, int64_t nc);
 rc_status xt2(rc_ctx* ctx, int64_t n, int64_t k, int64_t nc, const double* X, int64_t ldx, const double* T,
               int64_t ldt, double* Y, int64_t ldy, const double* W, int64_t ldw, const double* lam, int64_t res_count,

@@ -273,7 +273,7 @@ rc_status Solver::ritz_and_residuals(XtArgs a, int64_t s, int64_t res_count, voi
 // against (the deflation works on column-major blocks), outside the request server.
 bool Solver::rm_rr_ok(int64_t s, int64_t reps) const {
     return ctx_->rm_rr && dtype_ == RC_REAL64 && !ctx_->serve && P_.orth_mode == 0 && reps == 1 && foundSize_ == 0 &&
-           gram2_supported(dtype_, s) && xt2_supported(dtype_, s, s) && resid_supported(op_, s);
+           gram_dmma_supported(s, true) && resid_supported(op_, s);
 }
 
 rc_status Solver::r32_block(int64_t s, void** out) {
@@ -328,8 +328,7 @@ rc_status Solver::rr_fused(int64_t s, int64_t res_count, bool* ok, void* R32) {
         RC_TRY(rc_slot(ctx_, S_WRM, (size_t)n_ * ldrm * sizeof(double), &wrm));
         const double one[2] = {1.0, 0.0}, zero[2] = {0.0, 0.0};
         RC_TRY(rm_step(ctx_, op_, vf, nullptr, wrm, ldrm, s, one, zero, zero, RC_PREC_FP64));
-        RC_TRY(gram2(ctx_, n_, s, (const double*)vf, ldrm, (const double*)vf, ldrm, (double*)G_, (const double*)wrm,
-                     ldrm, (double*)H_, true));
+        RC_TRY(gram_dmma(ctx_, dtype_, n_, s, vf, ldrm, G_, wrm, ldrm, H_, true));
     } else {
         StepArgs st;
         st.s = s;
@@ -337,9 +336,8 @@ rc_status Solver::rr_fused(int64_t s, int64_t res_count, bool* ok, void* R32) {
         st.y = W_; st.yp = P64; st.ldy = n_;
         st.cp = P64;
         RC_TRY(op_step(ctx_, op_, st));
-        if (gram2_supported(dtype_, s)) {
-            RC_TRY(gram2(ctx_, n_, s, (const double*)V_, n_, (const double*)V_, n_, (double*)G_, (const double*)W_,
-                         n_, (double*)H_));
+        if (dtype_ == RC_REAL64 && gram_dmma_supported(s, false)) {
+            RC_TRY(gram_dmma(ctx_, dtype_, n_, s, V_, n_, G_, W_, n_, H_, false));
         } else {
             RC_TRY(gram(ctx_, dtype_, n_, s, s, V_, n_, V_, n_, G_, true));
             RC_TRY(gram(ctx_, dtype_, n_, s, s, V_, n_, W_, n_, H_, true));

@@ -144,6 +144,7 @@ xt_dmma_kernel(int64_t n, int k, int nc, const double* X, int64_t ldx, const dou
                         if (len & 1) {
                             if (k0 + lane == k - 1) {
                                 xd[lane * xpitch + len - 1] = src[len - 1];
+                                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
                                 --len;
                             } else {
                                 ++len;

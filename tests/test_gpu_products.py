@@ -48,3 +48,29 @@ def test_ritz_vectors_are_the_product_with_q(ctx, complex_, dims, s, pad):
     AV = (A @ out.T).T
     np.testing.assert_allclose(W, AV, rtol=0, atol=200 * EPS)
     np.testing.assert_allclose(res, np.linalg.norm(AV - w[:, None] * out, axis=1), rtol=0, atol=1e-12)
+
+
+@pytest.mark.parametrize("complex_", [False, True])
+@pytest.mark.parametrize("s", [1, 7, 8, 9, 17, 25, 33, 41, 49, 64, 65, 81, 96, 97, 129, 161, 192])
+@pytest.mark.parametrize("n,pad,shift", [(0, 0, 0), (1037, 0, 0), (1037, 1, 0), (20000, 1, 0), (1031, 2, 1)])
+def test_gram_tiles(ctx, complex_, s, n, pad, shift):
+    """Cholesky QR at every number of 8-column tiles, the fewest rows (n = s), leading dimensions even and odd, and
+    blocks that start 8 bytes (a complex entry) off: the factor of a QR with a positive diagonal. Two passes from a
+    random block (condition below 1e3 for n > s): an entry's error is a few s eps."""
+    import torch
+    rng = np.random.default_rng(100 * s + n)
+    n = n or s
+    V = rng.standard_normal((s, n)) + (1j * rng.standard_normal((s, n)) if complex_ else 0)
+    if n == s:
+        V += 4 * s * np.eye(s)
+    ld = n + pad
+    buf = torch.zeros(s * ld + 8, dtype=torch.complex128 if complex_ else torch.float64, device="cuda")
+    Vd = buf[shift:shift + s * ld].view(s, ld)
+    Vd[:, :n] = torch.from_numpy(V)
+    torch.cuda.synchronize()
+    R.cholqr(ctx, Vd, n, s, complex_, ld=ld)
+    out = Vd.cpu().numpy()
+    assert not out[:, n:].any()
+    q, r = np.linalg.qr(V.T)
+    ph = np.diag(r) / np.abs(np.diag(r))
+    np.testing.assert_allclose(out[:, :n], (q * ph).T, rtol=0, atol=1e-13)
