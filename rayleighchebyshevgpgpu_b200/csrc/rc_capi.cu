@@ -14,6 +14,7 @@
 #include "rc_common.cuh"
 #include "rc_cpoly.h"
 #include "rc_internal.h"
+#include "rc_tile.h"
 
 namespace rcb {
 rc_status solve(rc_ctx* ctx, rc_op* op, const rc_solve_params& p, const void* v0, double* evals_out, void* evecs_out,
@@ -98,6 +99,8 @@ static void op_release(rc_op* op) {
     if (op->colind) cudaFree(op->colind);
     if (op->vals64) cudaFree(op->vals64);
     if (op->vals32) cudaFree(op->vals32);
+    if (op->pack64) cudaFree(op->pack64);
+    if (op->pack32) cudaFree(op->pack32);
     if (op->diag64) cudaFree(op->diag64);
     if (op->diag32) cudaFree(op->diag32);
     if (op->phase64) cudaFree(op->phase64);
@@ -146,6 +149,7 @@ rc_status rc_ctx_create(int device, rc_ctx** out) {
         const int t = std::atoi(v) / 32 * 32;
         c->jacobi_threads = t >= 64 && t <= 1024 ? t : 0;
     }
+    if (const char* v = std::getenv("RCB200_TILE")) c->tile = std::max(0, std::min(2, std::atoi(v)));
     if (const char* v = std::getenv("RCB200_RM_RR")) c->rm_rr = std::atoi(v) != 0 ? 1 : 0;
     if (const char* v = std::getenv("RCB200_GRAM_C")) c->gram_c = std::atoi(v) != 0 ? 1 : 0;
     if (const char* v = std::getenv("RCB200_ROWS27W")) c->rows27w = std::atoi(v) != 0 ? 1 : 0;
@@ -231,6 +235,35 @@ static rc_status dev_copy(rc_ctx* ctx, void** dst, const void* src, size_t bytes
     return RC_OK;
 }
 
+// Whether the rows are those of a 7-point stencil on a grid: offsets 0, +-1, +-L, +-P with L | P | n, and row i holds
+// the diagonal and exactly the neighbours that lie in the grid, columns ascending. Sets op->gx, gy, gz.
+static void csr_grid(rc_op* op, const int32_t* rowptr, const int32_t* colind) {
+    const int64_t* o = op->offsets;
+    const int64_t L = o[5], P = o[6], n = op->n;
+    if (o[3] != 0 || o[4] != 1 || o[2] != -1 || L < 2 || o[1] != -L || o[0] != -P || P <= L || P % L || n % P) return;
+    const int64_t ny = P / L, nz = n / P;
+    int64_t i = 0;
+    for (int64_t z = 0; z < nz; ++z)
+        for (int64_t y = 0; y < ny; ++y)
+            for (int64_t x = 0; x < L; ++x, ++i) {
+                const int32_t* c = colind + rowptr[i];
+                const int32_t r = (int32_t)i;
+                int k = 0;
+                const int want = 1 + (z > 0) + (y > 0) + (x > 0) + (x + 1 < L) + (y + 1 < ny) + (z + 1 < nz);
+                if (rowptr[i + 1] - rowptr[i] != want) return;
+                if (z > 0 && c[k++] != r - P) return;
+                if (y > 0 && c[k++] != r - L) return;
+                if (x > 0 && c[k++] != r - 1) return;
+                if (c[k++] != r) return;
+                if (x + 1 < L && c[k++] != r + 1) return;
+                if (y + 1 < ny && c[k++] != r + L) return;
+                if (z + 1 < nz && c[k++] != r + P) return;
+            }
+    op->gx = L;
+    op->gy = ny;
+    op->gz = nz;
+}
+
 rc_status rc_op_csr_create(rc_ctx* ctx, int dtype, int64_t n, int64_t nnz, const int32_t* rowptr,
                            const int32_t* colind, const void* vals, rc_op** out) {
     RC_CHECK_CTX(ctx);
@@ -250,11 +283,18 @@ rc_status rc_op_csr_create(rc_ctx* ctx, int dtype, int64_t n, int64_t nnz, const
     int64_t band = 0;
     std::vector<int64_t> offs;  // distinct column offsets, while there are few
     bool few = true;
+    size_t at = 0;  // where the last offset was found: the next one usually follows it
     for (int64_t i = 0; i < n; ++i)
         for (int32_t k = rowptr[i]; k < rowptr[i + 1]; ++k) {
             const int64_t o = (int64_t)colind[k] - i;
             band = std::max<int64_t>(band, o);
-            if (few && std::find(offs.begin(), offs.end(), o) == offs.end()) {
+            if (!few) continue;
+            if (at + 1 < offs.size() && offs[at + 1] == o) {
+                ++at;
+                continue;
+            }
+            at = (size_t)(std::find(offs.begin(), offs.end(), o) - offs.begin());
+            if (at == offs.size()) {
                 offs.push_back(o);
                 few = (int)offs.size() <= rc_op::kMaxOffsets;
             }
@@ -273,10 +313,19 @@ rc_status rc_op_csr_create(rc_ctx* ctx, int dtype, int64_t n, int64_t nnz, const
         op->n_offsets = (int)offs.size();
         for (size_t q = 0; q < offs.size(); ++q) op->offsets[q] = offs[q];
     }
+    if (op->n_offsets == 7) csr_grid(op, rowptr, colind);
     const size_t vsz = (dtype == RC_COMPLEX128 ? 16 : 8);
     rc_status st = dev_copy(ctx, (void**)&op->rowptr, rowptr, (size_t)(n + 1) * 4, op);
     if (st == RC_OK) st = dev_copy(ctx, (void**)&op->colind, colind, (size_t)nnz * 4, op);
     if (st == RC_OK) st = dev_copy(ctx, &op->vals64, vals, (size_t)nnz * vsz, op);
+    if (st == RC_OK && op->gx > 0) {
+        size_t b = 0;
+        st = rcb::tile_pack(ctx, op, false, op->vals64, &op->pack64, &b);
+        if (st == RC_OK) {
+            op->bytes += (int64_t)b;
+            ctx->op_bytes += (int64_t)b;
+        }
+    }
     if (st != RC_OK) {
         rc_op_destroy(op);
         return st;

@@ -78,21 +78,27 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, unsigned parity) {
     return false;
 }
 
-// A tensor map of doubles: `inner` consecutive ones in each of `outer` rows, `ld` apart (ld even, p 16-byte
-// aligned), tiles of box_inner x box_outer, not swizzled. False when the driver refuses it.
-inline bool tma_map_2d(CUtensorMap* map, const double* p, int64_t inner, int64_t outer, int64_t ld, int box_inner,
-                       int box_outer) {
-    typedef CUresult (*Fn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
-                           const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
-                           CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-    static Fn fn = [] {  // through the runtime: no link-time dependency on libcuda
+// The driver's cuTensorMapEncodeTiled, through the runtime (no link-time dependency on libcuda), or null.
+typedef CUresult (*TensorMapEncodeFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
+                                      const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
+                                      CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+inline TensorMapEncodeFn tensor_map_encode() {
+    static TensorMapEncodeFn fn = [] {
         void* f = nullptr;
         cudaDriverEntryPointQueryResult q;
         if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &f, cudaEnableDefault, &q) != cudaSuccess ||
             q != cudaDriverEntryPointSuccess)
             f = nullptr;
-        return (Fn)f;
+        return (TensorMapEncodeFn)f;
     }();
+    return fn;
+}
+
+// A tensor map of doubles: `inner` consecutive ones in each of `outer` rows, `ld` apart (ld even, p 16-byte
+// aligned), tiles of box_inner x box_outer, not swizzled. False when the driver refuses it.
+inline bool tma_map_2d(CUtensorMap* map, const double* p, int64_t inner, int64_t outer, int64_t ld, int box_inner,
+                       int box_outer) {
+    const TensorMapEncodeFn fn = tensor_map_encode();
     if (!fn) return false;
     const cuuint64_t dims[2] = {(cuuint64_t)inner, (cuuint64_t)outer};
     const cuuint64_t strides[1] = {(cuuint64_t)ld * sizeof(double)};
@@ -100,6 +106,22 @@ inline bool tma_map_2d(CUtensorMap* map, const double* p, int64_t inner, int64_t
     return fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 2, const_cast<double*>(p), dims, strides, box, es,
               CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+// A tensor map of dense 4-D blocks of 32-bit words, dims[0] of them a multiple of 4 (what lies outside reads as zero).
+inline bool tma_map_words_4d(CUtensorMap* map, const void* p, const int64_t (&dims)[4], const int (&box)[4]) {
+    const TensorMapEncodeFn fn = tensor_map_encode();
+    if (!fn) return false;
+    cuuint64_t d[4], st[3];
+    cuuint32_t b[4], es[4] = {1, 1, 1, 1};
+    for (int k = 0; k < 4; ++k) {
+        d[k] = (cuuint64_t)dims[k];
+        b[k] = (cuuint32_t)box[k];
+        if (k < 3) st[k] = (k ? st[k - 1] : 4) * d[k];
+    }
+    return fn(map, CU_TENSOR_MAP_DATA_TYPE_INT32, 4, const_cast<void*>(p), d, st, b, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
+              CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) ==
+           CUDA_SUCCESS;
 }
 
 }  // namespace rcb

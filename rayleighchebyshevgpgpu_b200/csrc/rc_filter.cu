@@ -21,6 +21,7 @@
 #include <type_traits>
 #include "rc_common.cuh"
 #include "rc_internal.h"
+#include "rc_tile.h"
 
 namespace rcb {
 
@@ -351,6 +352,17 @@ rc_status ensure_fp32(rc_ctx* ctx, rc_op* op) {
         cvt_f64_f32_kernel<<<4 * kB200Sms, 256, 0, ctx->stream>>>((const double*)op->vals64, (float*)p, cnt);
         ctx->launches++;
         RC_CU(ctx, cudaGetLastError());
+        if (op->gx > 0) {
+            size_t b = 0;
+            const rc_status st = tile_pack(ctx, op, true, p, &op->pack32, &b);
+            if (st != RC_OK) {
+                cudaStreamSynchronize(ctx->stream);
+                cudaFree(p);
+                return st;
+            }
+            op->bytes += (int64_t)b;
+            ctx->op_bytes += (int64_t)b;
+        }
         op->vals32 = p;
         op->bytes += cnt * 4;
         ctx->op_bytes += cnt * 4;

@@ -21,6 +21,7 @@
 #include "rc_rowops.cuh"
 #include "rc_rmstep.cuh"
 #include "rc_staged.cuh"
+#include "rc_tile.h"
 
 namespace rcb {
 
@@ -147,6 +148,7 @@ struct StageOffsets {
     int n = 0;
     int64_t off[rc_op::kMaxOffsets] = {};
     int64_t max_row_nnz = 0;
+    const rc_op* op = nullptr;
 };
 
 static bool stage_offsets(const rc_op* op, StageOffsets* so) {
@@ -321,10 +323,31 @@ static bool try_staged(rc_ctx* ctx, const Pol& pol, const StageOffsets* so, int6
     }
 }
 
+template <class TC>
+static bool step_real(TC v) {
+    if constexpr (IsComplex<TC>::value) return v.y == 0;
+    else return true;
+}
+template <class TC>
+static double step_re(TC v) {
+    if constexpr (IsComplex<TC>::value) return (double)v.x;
+    else return (double)v;
+}
+
 template <class Pol, class TS, class TC, int W, class IX, bool SRC, class TM = TS>
 static void launch_step(rc_ctx* ctx, const Pol& pol, int64_t n, int nseg, int64_t ld, int groups, const TM* x,
                         const TM* z, TM* y, TC a, TC b, TC g, int64_t pf_z, int64_t pf_x, const TM* src,
                         const float* sig, const StageOffsets* so = nullptr) {
+    // large blocks of 7- and 27-point operators: from shared-memory tiles
+    constexpr bool kF64 = std::is_same<TM, double>::value || std::is_same<TM, double2>::value;
+    constexpr bool kBf16 = std::is_same<TM, __nv_bfloat16>::value || std::is_same<TM, __nv_bfloat162>::value;
+    if constexpr (SRC ? kBf16 : kF64) {
+        constexpr TileType type = IsComplex<TC>::value ? (SRC ? TT_BF16C : TT_C128) : (SRC ? TT_BF16 : TT_F64);
+        const bool real = step_real(a) && step_real(b) && step_real(g);
+        if (real && so && so->op && !ctx->staged && tile_supported(ctx, so->op, type, ld) &&
+            tile_step(ctx, so->op, type, ld, x, z, y, step_re(a), step_re(b), step_re(g), src, sig))
+            return;
+    }
     const int rows_per_iter = kRmThreads / nseg;
     if constexpr (IsStencil27<Pol>::value) {
         using TD = typename IsStencil27<Pol>::diag_t;
@@ -636,7 +659,9 @@ static rc_status rm_filter_dispatch(rc_ctx* ctx, rc_op* op, void* V, int64_t ldv
     const int64_t n = op->n;
     const int64_t band = op->kind == 0 ? op->band : (op->skind == 5 ? op->nx : op->nx * op->ny);
     StageOffsets so_v;
-    const StageOffsets* so = stage_offsets(op, &so_v) ? &so_v : nullptr;
+    stage_offsets(op, &so_v);
+    so_v.op = op;
+    const StageOffsets* so = &so_v;
     if (op->kind == 0) {
         const TS* vals = (const TS*)(sizeof(real_t<TS>) == 8 ? op->vals64 : op->vals32);
         CsrRows<TS, TC> pol{op->rowptr, op->colind, vals};
@@ -720,7 +745,9 @@ static rc_status rm_corr_dispatch(rc_ctx* ctx, rc_op* op, TV* V, int64_t ldv, in
     const int64_t n = op->n;
     const int64_t band = op->kind == 0 ? op->band : (op->skind == 5 ? op->nx : op->nx * op->ny);
     StageOffsets so_v;
-    const StageOffsets* so = stage_offsets(op, &so_v) ? &so_v : nullptr;
+    stage_offsets(op, &so_v);
+    so_v.op = op;
+    const StageOffsets* so = &so_v;
     if (op->kind == 0) {
         CsrRows<TS, TS> pol{op->rowptr, op->colind, (const TS*)op->vals32};
         return rm_corr_select<CsrRows<TS, TS>, TS>(ctx, pol, n, V, ldv, s, degree, a, b, R, sig, coef, A, B, ld, band,
@@ -824,7 +851,9 @@ static rc_status step_dispatch(rc_ctx* ctx, rc_op* op, int64_t ld, const void* x
     const int64_t n = op->n;
     const int64_t band = op->kind == 0 ? op->band : (op->skind == 5 ? op->nx : op->nx * op->ny);
     StageOffsets so_v;
-    const StageOffsets* so = stage_offsets(op, &so_v) ? &so_v : nullptr;
+    stage_offsets(op, &so_v);
+    so_v.op = op;
+    const StageOffsets* so = &so_v;
     if (op->kind == 0) {
         const TS* vals = (const TS*)(sizeof(real_t<TS>) == 8 ? op->vals64 : op->vals32);
         CsrRows<TS, TC> pol{op->rowptr, op->colind, vals};

@@ -92,6 +92,9 @@ struct rc_ctx {
     // for the FP64 SIMT kernel, from RCB200_GRAM_C.
     int gram_c = 1;
     int64_t jacobi_sweeps = 0;
+    // Degree steps and residual blocks of 7- and 27-point operators from shared-memory tiles (rc_tile.cu): 1
+    // (default: large blocks), 0 (never) or 2 (always), from RCB200_TILE.
+    int tile = 1;
     // Rayleigh-Ritz of the correction filter's output on row-major blocks (the filtered block and
     // W = A V formed row-major, no transposes): 1 (default) or 0, from RCB200_RM_RR.
     int rm_rr = 1;
@@ -142,6 +145,11 @@ struct rc_op {
     int32_t* colind = nullptr;
     void* vals64 = nullptr;
     void* vals32 = nullptr;  // built lazily for the mixed-precision filter
+    // 7-point structure: every row holds the diagonal and exactly its in-grid neighbours of a gx x gy x gz grid,
+    // columns ascending (0: not so). Then also the rows' weights, eight per row, for the tile kernels (rc_tile.cu).
+    int64_t gx = 0, gy = 0, gz = 0;
+    void* pack64 = nullptr;
+    void* pack32 = nullptr;
     // stencil
     int skind = 7;
     int64_t nx = 1, ny = 1, nz = 1;

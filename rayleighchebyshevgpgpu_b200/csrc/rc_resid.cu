@@ -15,6 +15,7 @@
 #include "rc_common.cuh"
 #include "rc_internal.h"
 #include "rc_rmstep.cuh"
+#include "rc_tile.h"
 
 namespace rcb {
 
@@ -385,6 +386,20 @@ rc_status resid_block(rc_ctx* ctx, const rc_op* op, const void* Yrm, int64_t ld,
     if (res_count < 0 || res_count > s || ld != rm_leading_dim(op->dtype, P64, s) ||
         (R && ldr != corr_leading_dim(op->dtype, s)))
         return rc_fail(ctx, RC_ERR_INVALID, "residual block: bad sizes");
+    double* part = nullptr;
+    int64_t parts = 0;
+    rc_status st = RC_OK;
+    if (tile_supported(ctx, op, op->dtype == RC_COMPLEX128 ? TT_C128 : TT_F64, ld) &&
+        tile_resid(ctx, op, Yrm, ld, s, lam, res_count, R, ldr, &part, &parts, &st)) {
+        RC_TRY(st);
+        RC_CU(ctx, cudaGetLastError());
+        if (res_count > 0) {
+            resid_norm_reduce_kernel<<<(unsigned)res_count, 256, 0, ctx->stream>>>(parts, (int)res_count, part, res);
+            ctx->launches++;
+            RC_CU(ctx, cudaGetLastError());
+        }
+        return RC_OK;
+    }
     if (op->dtype == RC_COMPLEX128)
         return resid_dispatch<double2>(ctx, op, (const double2*)Yrm, ld, s, lam, res_count, res, R, ldr);
     return resid_dispatch<double>(ctx, op, (const double*)Yrm, ld, s, lam, res_count, res, R, ldr);

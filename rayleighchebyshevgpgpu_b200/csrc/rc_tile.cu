@@ -1,0 +1,749 @@
+// rc_tile.cu -- degree steps and residual blocks of 7- and 27-point operators on large row-major blocks, from
+// tiles in shared memory.
+//
+// Rows are the points of a grid, i = x + nx (y + ny z); a matrix in CSR form takes part when its rows hold exactly
+// the in-grid neighbours of such a grid (op->gx, found when the operator is created). A CTA takes tiles of tx x ty
+// points and a panel of up to 12 16-byte slices of their columns, and marches along z. One producer warp brings
+// the planes of x (with a halo of one point: what lies outside the grid reads as zero), of x_{k-2} and the source
+// block, and of the rows' weights into rings of shared-memory slots, one TMA tile copy each; the other warps
+// wait for the slots they read (rc_dmma.cuh). A thread owns one slice of four points in a line along y: it reads
+// the line's six points once for the y neighbours of all four, two x neighbours each and the point above, and
+// keeps the point below in registers. 27 points: the sums over three points along x of the six lines give the
+// 3x3 sums of all four rows, which are kept for the planes above and below.
+//
+// The gather kernels (rc_filter_rm.cu, rc_resid.cu) read every neighbour through L1 for each thread: at 128^3 with
+// 96 bfloat16 columns their loads and fills take 78 % of the L1 data cycles and 68 % of the issue slots, and a CSR
+// row's index loads add to both; DRAM then runs at 0.7 of its rate. Here a row's neighbours cost 4.5 shared-memory
+// reads instead of 8 (27 points: 4.5 instead of 9), no address or bounds arithmetic per neighbour, and nothing
+// waits on DRAM but the producer. The sums are formed in the gather kernels' order (5- and 7-point: the same bits).
+//
+// Units (a panel of a tile over ml planes) are taken in turn by one CTA per SM, panels fastest, then x, y, z: the
+// tiles in flight are neighbours, so a halo's rows are read from DRAM once. ml is chosen so that the last turn is
+// nearly full (tile_plan).
+#include <algorithm>
+#include <type_traits>
+#include "rc_common.cuh"
+#include "rc_dmma.cuh"
+#include "rc_internal.h"
+#include "rc_rmstep.cuh"
+#include "rc_tile.h"
+
+namespace rcb {
+
+namespace {
+
+// Smallest block (bytes) for which the tile kernels are taken.
+constexpr int64_t kTileMinBytes = 32ll << 20;
+
+enum { TK_STENCIL7 = 0, TK_CSR7 = 1, TK_STENCIL27 = 2 };
+constexpr int TL_ROWS = 4;          // points along y per thread
+constexpr int TL_MAX_SLOTS = 4;
+constexpr int TL_MAX_SEG = 12;      // slices per panel, at most
+constexpr int TL_THREADS = 384;     // product threads, at most
+
+// What a kernel needs beside the maps. Sizes in bytes; slots are multiples of 128.
+struct TileArgs {
+    int nx, ny, nz, tx, ty, ltx;    // ltx: log2 of tx
+    int ntx, nty, ml, nml;          // tiles along x and y, planes per unit, units along z
+    int panels, nseg, slices;       // slices per panel and per row
+    int units;
+    int64_t ld;                     // elements per row
+    int xslots, zslots, xbytes, zbytes, cbytes;
+    int zops;                       // planes per z slot: x_{k-2} and / or the source block
+    int has_z;
+    double off;                     // stencils: every neighbour's weight, the diagonal and (complex) the phases
+    const void* diag;
+    const void* phase;
+};
+
+template <class TM, class TC>
+struct TileStep {
+    TM* y;
+    const float* sig;
+    TC alpha, beta, gamma;
+};
+struct TileResid {
+    const double* lam;
+    double* part;                   // [CTA][res_count]
+    void* R;                        // row-major bfloat16 (rc_corr_t / rc_corr2_t), or null
+    int64_t ldr;
+    int res_count;
+    int64_t s;
+};
+struct TileMaps {
+    CUtensorMap x, z, src, co;
+};
+
+__device__ __forceinline__ void tma_load_4d(uint32_t dst, const CUtensorMap* map, int c, int x, int y, int z,
+                                            uint32_t bar) {
+    asm volatile(
+        "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], "
+        "[%6];" ::"r"(dst),
+        "l"(map), "r"(c), "r"(x), "r"(y), "r"(z), "r"(bar)
+        : "memory");
+}
+
+struct Unit {
+    int panel, x0, y0, m0, m1;
+};
+__device__ __forceinline__ Unit tile_unit(const TileArgs& A, int u) {
+    Unit U;
+    U.panel = u % A.panels;
+    int t = u / A.panels;
+    U.x0 = (t % A.ntx) * A.tx;
+    t /= A.ntx;
+    U.y0 = (t % A.nty) * A.ty;
+    U.m0 = (t / A.nty) * A.ml;
+    U.m1 = min(A.nz, U.m0 + A.ml);
+    return U;
+}
+
+// The ring positions of one side (producer or product warp).
+struct Ring {
+    int slot = 0;
+    unsigned ph = 0;
+    __device__ __forceinline__ void next(int slots) {
+        if (++slot == slots) {
+            slot = 0;
+            ph ^= 1;
+        }
+    }
+};
+
+template <class TS, class TC, class TM>
+struct TileVec {
+    static constexpr int V = Slice<TS, TM>::V;
+    // a += c x in the gather kernels' rounding (packed FP32 pairs for bfloat16 blocks)
+    __device__ static __forceinline__ void add(TC (&a)[V], TC c, const uint4& u) {
+        const Slice<TS, TM> p = slice_from<TS, TM>(u);
+        if constexpr (sizeof(TM) == 2) {
+#pragma unroll
+            for (int v = 0; v < V; v += 2) ffma2(c, c, p.v[v], p.v[v + 1], a[v], a[v + 1]);
+        } else {
+#pragma unroll
+            for (int v = 0; v < V; ++v) a[v] = s_fma(c, s_cvt<TC>(p.v[v]), a[v]);
+        }
+    }
+};
+
+// One row of weights in shared memory: -P, -L, -1, 0, 1, L, P, (unused).
+template <class TC>
+struct RowWeights {
+    TC w[8];
+};
+
+template <int KIND, class TS, class TC, class TM, bool SRC, bool RESID>
+__global__ void __launch_bounds__(TL_THREADS + 32, 1)
+tile_kernel(TileArgs A, const __grid_constant__ TileMaps M, TileStep<TM, TC> S, TileResid Q) {
+    constexpr int V = Slice<TS, TM>::V;
+    constexpr bool CPLX = IsComplex<TC>::value;
+    using TD = real_t<TC>;
+    using Vec = TileVec<TS, TC, TM>;
+    extern __shared__ __align__(128) unsigned char tls[];
+    __shared__ __align__(8) uint64_t bars[4 * TL_MAX_SLOTS];
+    const int tid = threadIdx.x, lane = tid & 31, nt = blockDim.x - 32;
+    const uint32_t xfull = smem_u32(bars), xempty = xfull + 8 * TL_MAX_SLOTS, zfull = xempty + 8 * TL_MAX_SLOTS,
+                   zempty = zfull + 8 * TL_MAX_SLOTS;
+    const bool zring = A.zops > 0 || KIND == TK_CSR7;
+    const int zslot = A.zops * A.zbytes + A.cbytes;
+    unsigned char* xs0 = tls;
+    unsigned char* zs0 = tls + A.xslots * A.xbytes;
+    if (tid == 0) {
+        for (int s = 0; s < A.xslots; ++s) {
+            mbar_init(xfull + 8 * s, 1);
+            mbar_init(xempty + 8 * s, nt / 32);
+        }
+        for (int s = 0; s < A.zslots; ++s) {
+            mbar_init(zfull + 8 * s, 1);
+            mbar_init(zempty + 8 * s, nt / 32);
+        }
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    __syncthreads();
+    Ring rx, rz;
+    if (tid >= nt) {  // the producer: planes m0 - 1, m0, then m + 1 of x with the rest of plane m
+        if (lane != 0) return;
+        const int cw = A.nseg * 4;  // 32-bit words of a panel's row
+        const unsigned xtx = (unsigned)(A.nseg * 16 * (A.tx + 2) * (A.ty + 2));
+        const unsigned ztx = (unsigned)(A.zops * A.nseg * 16 * A.tx * A.ty) +
+                             (KIND == TK_CSR7 ? (unsigned)(sizeof(RowWeights<TC>) * A.tx * A.ty) : 0u);
+        int64_t nxl = 0, nzl = 0;
+        bool ok = true;
+        auto load_x = [&](const Unit& U, int m) {
+            if (nxl >= A.xslots && !mbar_wait(xempty + 8 * rx.slot, rx.ph ^ 1)) return false;
+            const uint32_t bar = xfull + 8 * rx.slot;
+            mbar_arrive_tx(bar, xtx);
+            tma_load_4d(smem_u32(xs0 + rx.slot * A.xbytes), &M.x, U.panel * cw, U.x0 - 1, U.y0 - 1, m, bar);
+            rx.next(A.xslots);
+            ++nxl;
+            return true;
+        };
+        auto load_z = [&](const Unit& U, int m) {
+            if (nzl >= A.zslots && !mbar_wait(zempty + 8 * rz.slot, rz.ph ^ 1)) return false;
+            const uint32_t bar = zfull + 8 * rz.slot;
+            unsigned char* d = zs0 + rz.slot * zslot;
+            mbar_arrive_tx(bar, ztx);
+            if (A.has_z) tma_load_4d(smem_u32(d), &M.z, U.panel * cw, U.x0, U.y0, m, bar);
+            if (SRC) tma_load_4d(smem_u32(d + (A.zops - 1) * A.zbytes), &M.src, U.panel * cw, U.x0, U.y0, m, bar);
+            if (KIND == TK_CSR7) tma_load_4d(smem_u32(d + A.zops * A.zbytes), &M.co, 0, U.x0, U.y0, m, bar);
+            rz.next(A.zslots);
+            ++nzl;
+            return true;
+        };
+        for (int u = blockIdx.x; u < A.units && ok; u += gridDim.x) {
+            const Unit U = tile_unit(A, u);
+            ok = load_x(U, U.m0 - 1) && load_x(U, U.m0);
+            for (int m = U.m0; m < U.m1 && ok; ++m) ok = load_x(U, m + 1) && (!zring || load_z(U, m));
+        }
+        // copies still in flight land before the CTA ends
+        for (int s = 0; s < A.xslots && s < nxl; ++s) {
+            if (--rx.slot < 0) {
+                rx.slot = A.xslots - 1;
+                rx.ph ^= 1;
+            }
+            if (!mbar_wait(xfull + 8 * rx.slot, rx.ph)) break;
+        }
+        for (int s = 0; s < A.zslots && s < nzl; ++s) {
+            if (--rz.slot < 0) {
+                rz.slot = A.zslots - 1;
+                rz.ph ^= 1;
+            }
+            if (!mbar_wait(zfull + 8 * rz.slot, rz.ph)) break;
+        }
+        return;
+    }
+
+    const int row = tid / A.nseg, seg = tid - row * A.nseg;
+    const int lx = row & (A.tx - 1), ly = (row >> A.ltx) * TL_ROWS;
+    const int cb = A.nseg * 16, xp = (A.tx + 2) * cb;          // bytes of a point and of a line of the x tile
+    const int xo = ly * xp + (lx + 1) * cb + seg * 16;         // line ly - 1 (halo) of this thread's column
+    const int zo = (ly * A.tx + lx) * cb + seg * 16, zp = A.tx * cb;
+    const TD* diag = (const TD*)A.diag;
+    double sq[RESID ? V : 1];
+#pragma unroll
+    for (int v = 0; v < (RESID ? V : 1); ++v) sq[v] = 0.0;
+    bool ok = true;
+    for (int u = blockIdx.x; u < A.units && ok; u += gridDim.x) {
+        const Unit U = tile_unit(A, u);
+        const int gx = U.x0 + lx, gy = U.y0 + ly;
+        const int slice = U.panel * A.nseg + seg;
+        const bool col_on = slice < A.slices && gx < A.nx;
+        const int nrow = col_on ? max(0, min(TL_ROWS, A.ny - gy)) : 0;
+        const int64_t col = (int64_t)slice * V;
+        const int64_t i0 = gx + (int64_t)A.nx * gy, plane = (int64_t)A.nx * A.ny;
+        float sg[SRC ? V : 1];
+        if (SRC) {
+#pragma unroll
+            for (int v = 0; v < V; ++v) sg[v] = col_on ? __ldg(S.sig + col + v) : 0.0f;
+        }
+        double lam[RESID ? V : 1];
+        if (RESID) {
+#pragma unroll
+            for (int v = 0; v < V; ++v) lam[v] = col + v < Q.s ? Q.lam[col + v] : 0.0;
+        }
+        const TC off = s_from<TC>(A.off, 0.0);
+        TC wm = off, wp = off;
+        if constexpr (CPLX && KIND == TK_STENCIL7) {
+            const TC p = col_on ? ((const TC*)A.phase)[gx] : off;
+            wm = s_mul(off, p);
+            wp = s_mul(off, s_conj(p));
+        }
+        // stencils: the diagonal of the next plane's points, fetched a plane ahead
+        TD dn[TL_ROWS];
+        auto fetch_diag = [&](int m) {
+            if constexpr (KIND != TK_CSR7) {
+#pragma unroll
+                for (int k = 0; k < TL_ROWS; ++k)
+                    dn[k] = k < nrow && m < U.m1 ? __ldg(diag + i0 + (int64_t)k * A.nx + (int64_t)m * plane) : TD(0);
+            }
+        };
+        fetch_diag(U.m0);
+        // the finished sums a (A x, or the box sum) of point k of plane m, whose own value is xi
+        auto finish = [&](int m, int k, const TC (&a)[V], const uint4& xr, const unsigned char* zb) {
+            const Slice<TS, TM> xi = slice_from<TS, TM>(xr);
+            const int64_t i = i0 + (int64_t)k * A.nx + (int64_t)m * plane;
+            if constexpr (RESID) {
+                if (k >= nrow) return;
+                float rv[2] = {0.0f, 0.0f};
+#pragma unroll
+                for (int v = 0; v < V; ++v) {
+                    if constexpr (CPLX) {
+                        double2 d = make_double2(fma(-lam[v], xi.v[v].x, a[v].x), fma(-lam[v], xi.v[v].y, a[v].y));
+                        if (col + v >= Q.s) d = make_double2(0.0, 0.0);
+                        sq[v] = fma(d.y, d.y, fma(d.x, d.x, sq[v]));
+                        rv[0] = (float)d.x;
+                        rv[1] = (float)d.y;
+                    } else {
+                        const double d = col + v < Q.s ? fma(-lam[v], xi.v[v], a[v]) : 0.0;
+                        sq[v] = fma(d, d, sq[v]);
+                        rv[v] = (float)d;
+                    }
+                }
+                if (Q.R) {
+                    using TR = typename std::conditional<CPLX, rc_corr2_t, rc_corr_t>::type;
+                    void* R = (TR*)Q.R + i * Q.ldr + col;
+                    if constexpr (sizeof(rc_corr_t) == 2) *(__nv_bfloat162*)R = __floats2bfloat162_rn(rv[0], rv[1]);
+                    else *(float2*)R = make_float2(rv[0], rv[1]);
+                }
+            } else {
+                Slice<TS, TM> zi{}, si{}, out;
+                if (A.has_z) zi = slice_from<TS, TM>(*reinterpret_cast<const uint4*>(zb + zo + k * zp));
+                if (SRC) si = slice_from<TS, TM>(*reinterpret_cast<const uint4*>(zb + (A.zops - 1) * A.zbytes + zo + k * zp));
+                if constexpr (sizeof(TM) == 2) {
+#pragma unroll
+                    for (int v = 0; v < V; v += 2) {
+                        float r0, r1;
+                        fmul2(S.alpha, S.alpha, a[v], a[v + 1], r0, r1);
+                        ffma2(S.beta, S.beta, xi.v[v], xi.v[v + 1], r0, r1);
+                        if (A.has_z) ffma2(S.gamma, S.gamma, zi.v[v], zi.v[v + 1], r0, r1);
+                        if (SRC) ffma2(sg[v], sg[v + 1], si.v[v], si.v[v + 1], r0, r1);
+                        out.v[v] = r0;
+                        out.v[v + 1] = r1;
+                    }
+                } else if constexpr (SRC && CPLX) {
+#pragma unroll
+                    for (int v = 0; v < V; ++v) {
+                        float r0, r1;
+                        fmul2(S.alpha.x, S.alpha.x, a[v].x, a[v].y, r0, r1);
+                        ffma2(S.beta.x, S.beta.x, xi.v[v].x, xi.v[v].y, r0, r1);
+                        if (A.has_z) ffma2(S.gamma.x, S.gamma.x, zi.v[v].x, zi.v[v].y, r0, r1);
+                        ffma2(sg[v], sg[v], si.v[v].x, si.v[v].y, r0, r1);
+                        out.v[v] = make_float2(r0, r1);
+                    }
+                } else {
+#pragma unroll
+                    for (int v = 0; v < V; ++v) {
+                        TC r = s_mul(S.alpha, a[v]);
+                        r = s_fma(S.beta, s_cvt<TC>(xi.v[v]), r);
+                        if (A.has_z) r = s_fma(S.gamma, s_cvt<TC>(zi.v[v]), r);
+                        out.v[v] = s_cvt<TS>(r);
+                    }
+                }
+                if (k < nrow) stv_once<TS, TM>(S.y + i * A.ld + col, out);
+            }
+        };
+        auto wait_x = [&]() {
+            ok = ok && mbar_wait(xfull + 8 * rx.slot, rx.ph);
+            return xs0 + rx.slot * A.xbytes + xo;
+        };
+        auto free_x = [&](int slot) {
+            __syncwarp();
+            if (lane == 0) mbar_arrive(xempty + 8 * slot);
+        };
+        auto ld16 = [](const unsigned char* p) { return *reinterpret_cast<const uint4*>(p); };
+        const unsigned char* zb = nullptr;
+        auto wait_z = [&]() {
+            if (!zring) return;
+            ok = ok && mbar_wait(zfull + 8 * rz.slot, rz.ph);
+            zb = zs0 + rz.slot * zslot;
+        };
+        auto free_z = [&]() {
+            if (!zring) return;
+            __syncwarp();
+            if (lane == 0) mbar_arrive(zempty + 8 * rz.slot);
+            rz.next(A.zslots);
+        };
+        if constexpr (KIND == TK_STENCIL27) {
+            // 3x3 sums of the four points in one plane, and their own values
+            auto plane_sums = [&](const unsigned char* p, TC (&b)[TL_ROWS][V], uint4 (&own)[TL_ROWS]) {
+#pragma unroll
+                for (int l = 0; l < TL_ROWS + 2; ++l) {
+                    const uint4 c = ld16(p + l * xp);
+                    const Slice<TS, TM> cl = slice_from<TS, TM>(ld16(p + l * xp - cb)), cc = slice_from<TS, TM>(c),
+                                        cr = slice_from<TS, TM>(ld16(p + l * xp + cb));
+                    if (l >= 1 && l <= TL_ROWS) own[l - 1] = c;
+                    TC t[V];
+#pragma unroll
+                    for (int v = 0; v < V; ++v) t[v] = s_add(s_add(s_cvt<TC>(cl.v[v]), s_cvt<TC>(cc.v[v])), s_cvt<TC>(cr.v[v]));
+#pragma unroll
+                    for (int k = l - 2; k <= l; ++k) {
+                        if (k < 0 || k >= TL_ROWS) continue;
+#pragma unroll
+                        for (int v = 0; v < V; ++v) b[k][v] = k == l ? t[v] : s_add(b[k][v], t[v]);
+                    }
+                }
+            };
+            TC s2[TL_ROWS][V], p0[TL_ROWS][V];  // sums of the planes below and here; of this plane
+            uint4 own[TL_ROWS];
+            {
+                plane_sums(wait_x(), s2, own);
+                free_x(rx.slot);
+                rx.next(A.xslots);
+                plane_sums(wait_x(), p0, own);
+                free_x(rx.slot);
+                rx.next(A.xslots);
+#pragma unroll
+                for (int k = 0; k < TL_ROWS; ++k)
+#pragma unroll
+                    for (int v = 0; v < V; ++v) s2[k][v] = s_add(s2[k][v], p0[k][v]);
+            }
+            for (int m = U.m0; m < U.m1 && ok; ++m) {
+                TD d[TL_ROWS];
+#pragma unroll
+                for (int k = 0; k < TL_ROWS; ++k) d[k] = dn[k];
+                fetch_diag(m + 1);
+                TC p1[TL_ROWS][V];
+                uint4 own1[TL_ROWS];
+                plane_sums(wait_x(), p1, own1);
+                free_x(rx.slot);
+                rx.next(A.xslots);
+                wait_z();
+#pragma unroll
+                for (int k = 0; k < TL_ROWS; ++k) {
+                    const TC dm = s_sub(s_from<TC>((double)d[k], 0.0), off);
+                    const Slice<TS, TM> xi = slice_from<TS, TM>(own[k]);
+                    TC a[V];
+#pragma unroll
+                    for (int v = 0; v < V; ++v)
+                        a[v] = s_fma(off, s_add(s2[k][v], p1[k][v]), s_mul(dm, s_cvt<TC>(xi.v[v])));
+                    finish(m, k, a, own[k], zb);
+                    own[k] = own1[k];
+#pragma unroll
+                    for (int v = 0; v < V; ++v) {
+                        s2[k][v] = s_add(p0[k][v], p1[k][v]);
+                        p0[k][v] = p1[k][v];
+                    }
+                }
+                free_z();
+            }
+        } else {
+            uint4 um[TL_ROWS];  // the points below
+            {
+                const unsigned char* p = wait_x();
+#pragma unroll
+                for (int k = 0; k < TL_ROWS; ++k) um[k] = ld16(p + (k + 1) * xp);
+                free_x(rx.slot);
+                rx.next(A.xslots);
+            }
+            const unsigned char* pc = wait_x();
+            int sc = rx.slot;
+            rx.next(A.xslots);
+            for (int m = U.m0; m < U.m1 && ok; ++m) {
+                TD d[TL_ROWS];
+                if constexpr (KIND == TK_STENCIL7) {
+#pragma unroll
+                    for (int k = 0; k < TL_ROWS; ++k) d[k] = dn[k];
+                    fetch_diag(m + 1);
+                }
+                const unsigned char* pn = wait_x();
+                wait_z();
+                uint4 c0 = ld16(pc), c1 = ld16(pc + xp);
+#pragma unroll
+                for (int k = 0; k < TL_ROWS; ++k) {
+                    const uint4 c2 = ld16(pc + (k + 2) * xp);
+                    const uint4 cl = ld16(pc + (k + 1) * xp - cb), cr = ld16(pc + (k + 1) * xp + cb);
+                    const uint4 cn = ld16(pn + (k + 1) * xp);
+                    TC a[V];
+#pragma unroll
+                    for (int v = 0; v < V; ++v) a[v] = s_zero(TC());
+                    if constexpr (KIND == TK_STENCIL7) {
+                        Vec::add(a, s_from<TC>((double)d[k], 0.0), c1);
+                        Vec::add(a, off, um[k]);
+                        Vec::add(a, wm, c0);
+                        Vec::add(a, off, cl);
+                        Vec::add(a, off, cr);
+                        Vec::add(a, wp, c2);
+                        Vec::add(a, off, cn);
+                    } else {
+                        const RowWeights<TC>& w = *reinterpret_cast<const RowWeights<TC>*>(
+                            zb + A.zops * A.zbytes + ((ly + k) * A.tx + lx) * sizeof(RowWeights<TC>));
+                        Vec::add(a, w.w[0], um[k]);
+                        Vec::add(a, w.w[1], c0);
+                        Vec::add(a, w.w[2], cl);
+                        Vec::add(a, w.w[3], c1);
+                        Vec::add(a, w.w[4], cr);
+                        Vec::add(a, w.w[5], c2);
+                        Vec::add(a, w.w[6], cn);
+                    }
+                    finish(m, k, a, c1, zb);
+                    um[k] = c1;
+                    c0 = c1;
+                    c1 = c2;
+                }
+                free_x(sc);
+                free_z();
+                pc = pn;
+                sc = rx.slot;
+                rx.next(A.xslots);
+            }
+            free_x(sc);
+        }
+    }
+    if constexpr (!RESID) {
+        // a plane that never landed: NaN to the caller
+        if (!ok) {
+            Slice<TS, TM> bad;
+#pragma unroll
+            for (int v = 0; v < V; ++v) bad.v[v] = s_from<TS>(__longlong_as_double(0x7ff8000000000000ll), 0.0);
+            stv<TS, TM>(S.y, bad);
+        }
+    } else if (Q.res_count > 0) {
+        // column sums over the CTA's points, rows in order (the panel is the same in all its units)
+        if (!ok) sq[0] = __longlong_as_double(0x7ff8000000000000ll);
+        asm volatile("bar.sync 1, %0;" ::"r"(nt) : "memory");
+        double* red = reinterpret_cast<double*>(tls);  // every slot has been read
+        const int pw = A.nseg * V, rows = nt / A.nseg;
+#pragma unroll
+        for (int v = 0; v < V; ++v) red[row * pw + seg * V + v] = sq[v];
+        asm volatile("bar.sync 1, %0;" ::"r"(nt) : "memory");
+        const int c0 = (blockIdx.x % A.panels) * pw;
+        for (int c = tid; c < Q.res_count; c += nt) {
+            double t = 0.0;
+            if (c >= c0 && c < c0 + pw)
+                for (int r = 0; r < rows; ++r) t += red[r * pw + c - c0];
+            Q.part[(int64_t)blockIdx.x * Q.res_count + c] = t;
+        }
+    }
+}
+
+// Rows of the 7-point CSR structure: weights by neighbour, zeros where there is none.
+template <class T>
+__global__ void tile_pack_kernel(int64_t n, int nx, int ny, int nz, const int32_t* __restrict__ rowptr,
+                                 const T* __restrict__ vals, RowWeights<T>* __restrict__ out) {
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t l = i / nx;
+        const int x = (int)(i - l * nx), z = (int)(l / ny), y = (int)(l - (int64_t)z * ny);
+        int k = rowptr[i];
+        RowWeights<T> w;
+        w.w[0] = z > 0 ? vals[k++] : s_zero(T());
+        w.w[1] = y > 0 ? vals[k++] : s_zero(T());
+        w.w[2] = x > 0 ? vals[k++] : s_zero(T());
+        w.w[3] = vals[k++];
+        w.w[4] = x + 1 < nx ? vals[k++] : s_zero(T());
+        w.w[5] = y + 1 < ny ? vals[k++] : s_zero(T());
+        w.w[6] = z + 1 < nz ? vals[k++] : s_zero(T());
+        w.w[7] = s_zero(T());
+        out[i] = w;
+    }
+}
+
+struct Structure {
+    int kind = -1;
+    int64_t nx = 0, ny = 0, nz = 0;
+};
+Structure structure(const rc_op* op, bool fp32) {
+    Structure S;
+    if (op->kind == 1 && (op->skind == 7 || op->skind == 27)) {
+        S.kind = op->skind == 7 ? TK_STENCIL7 : TK_STENCIL27;
+        S.nx = op->nx;
+        S.ny = op->ny;
+        S.nz = op->nz;
+    } else if (op->kind == 0 && op->gx > 0 && (fp32 ? op->pack32 : op->pack64)) {
+        S.kind = TK_CSR7;
+        S.nx = op->gx;
+        S.ny = op->gy;
+        S.nz = op->gz;
+    }
+    return S;
+}
+constexpr int tile_elem(TileType t) { return t == TT_BF16 ? 2 : (t == TT_BF16C ? 4 : (t == TT_F64 ? 8 : 16)); }
+
+// Tiles, slots and units for blocks of `slices` 16-byte slices a row; zops planes beside x, wbytes of weights a row.
+bool tile_plan(const rc_ctx* ctx, const Structure& S, int slices, int zops, int wbytes, TileArgs* out, unsigned* grid,
+               size_t* smem) {
+    TileArgs A = {};
+    A.nx = (int)S.nx;
+    A.ny = (int)S.ny;
+    A.nz = (int)S.nz;
+    A.slices = slices;
+    A.panels = (slices + TL_MAX_SEG - 1) / TL_MAX_SEG;
+    A.nseg = (slices + A.panels - 1) / A.panels;
+    A.tx = A.nseg > 3 ? 16 : 32;
+    A.ltx = A.nseg > 3 ? 4 : 5;
+    A.ty = A.nseg > 6 ? 8 : 16;
+    A.zops = zops;
+    auto up = [](int b) { return (b + 127) / 128 * 128; };
+    A.xbytes = up(A.nseg * 16 * (A.tx + 2) * (A.ty + 2));
+    A.zbytes = up(A.nseg * 16 * A.tx * A.ty);
+    A.cbytes = up(wbytes * A.tx * A.ty);
+    const int zslot = zops * A.zbytes + A.cbytes;
+    const int room = (int)ctx->smem_optin - 2048;
+    A.zslots = zslot ? 2 : 1;
+    A.xslots = std::min(TL_MAX_SLOTS, (room - A.zslots * zslot) / A.xbytes);
+    if (A.xslots < 3) return false;
+    if (zslot && A.xslots == TL_MAX_SLOTS && 3 * zslot + A.xslots * A.xbytes <= room) A.zslots = 3;
+    A.ntx = (A.nx + A.tx - 1) / A.tx;
+    A.nty = (A.ny + A.ty - 1) / A.ty;
+    const int64_t columns = (int64_t)A.panels * A.ntx * A.nty;
+    const int64_t ctas = std::max<int64_t>(1, ctx->sm_count / A.panels) * A.panels;
+    if (columns * A.nz > INT32_MAX) return false;
+    // planes per unit: the fewest turns x planes read (two more of x per unit, about the cost of one plane)
+    double best = 1e300;
+    for (int k = 1; k <= A.nz; ++k) {
+        const int ml = (A.nz + k - 1) / k;
+        const int64_t units = columns * ((A.nz + ml - 1) / ml);
+        const double cost = (double)((units + ctas - 1) / ctas) * (ml + 1.2);
+        if (cost < best) {
+            best = cost;
+            A.ml = ml;
+        }
+        if (ml <= 4) break;
+    }
+    A.nml = (A.nz + A.ml - 1) / A.ml;
+    A.units = (int)(columns * A.nml);
+    *grid = (unsigned)std::min<int64_t>(ctas, A.units);
+    // a CTA keeps its panel: whole turns of the panels
+    *grid = *grid / A.panels * A.panels;
+    const int red = A.tx * A.ty / TL_ROWS * A.nseg * 2 * 8;  // the residual's column sums
+    *smem = (size_t)std::max(A.xslots * A.xbytes + A.zslots * zslot, red);
+    *out = A;
+    return true;
+}
+
+bool tile_map(CUtensorMap* map, const void* p, const Structure& S, int64_t words, int bw, int bx, int by) {
+    const int64_t dims[4] = {words, S.nx, S.ny, S.nz};
+    const int box[4] = {bw, bx, by, 1};
+    return tma_map_words_4d(map, p, dims, box);
+}
+
+template <int KIND, class TS, class TC, class TM, bool SRC, bool RESID>
+bool tile_launch(rc_ctx* ctx, const TileArgs& A, const TileMaps& M, const TileStep<TM, TC>& S, const TileResid& Q,
+                 unsigned grid, size_t smem) {
+    auto kern = tile_kernel<KIND, TS, TC, TM, SRC, RESID>;
+    if (allow_max_smem(ctx, kern) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    const int nt = A.tx * A.ty / TL_ROWS * A.nseg;
+    kern<<<grid, nt + 32, smem, ctx->stream>>>(A, M, S, Q);
+    ctx->launches++;
+    return true;
+}
+
+}  // namespace
+
+bool tile_supported(const rc_ctx* ctx, const rc_op* op, TileType type, int64_t ld) {
+    if (!ctx->tile) return false;
+    const Structure S = structure(op, type == TT_BF16 || type == TT_BF16C);
+    if (S.kind < 0 || (op->dtype == RC_COMPLEX128) != (type == TT_C128 || type == TT_BF16C)) return false;
+    if (S.kind == TK_STENCIL27 && op->dtype == RC_COMPLEX128) return false;
+    return ctx->tile > 1 || op->n * ld * tile_elem(type) >= kTileMinBytes;
+}
+
+template <class TS, class TC, class TM, bool SRC>
+static bool tile_step_t(rc_ctx* ctx, const rc_op* op, TileType type, int64_t ld, const void* x, const void* z, void* y,
+                        double alpha, double beta, double gamma, const void* src, const float* sig) {
+    const bool fp32 = sizeof(real_t<TC>) == 4;
+    const Structure st = structure(op, fp32);
+    TileArgs A;
+    unsigned grid;
+    size_t smem;
+    const int zops = (z ? 1 : 0) + (SRC ? 1 : 0);
+    const int wb = st.kind == TK_CSR7 ? (int)sizeof(RowWeights<TC>) : 0;
+    const int64_t words = ld * (int64_t)sizeof(TM) / 4;
+    if (!tile_plan(ctx, st, (int)(words / 4), zops, wb, &A, &grid, &smem)) return false;
+    A.ld = ld;
+    A.has_z = z != nullptr;
+    A.off = op->offdiag;
+    A.diag = fp32 ? (const void*)op->diag32 : (const void*)op->diag64;
+    A.phase = fp32 ? op->phase32 : op->phase64;
+    TileMaps M = {};
+    bool ok = tile_map(&M.x, x, st, words, A.nseg * 4, A.tx + 2, A.ty + 2);
+    if (z) ok = ok && tile_map(&M.z, z, st, words, A.nseg * 4, A.tx, A.ty);
+    if (SRC) ok = ok && tile_map(&M.src, src, st, words, A.nseg * 4, A.tx, A.ty);
+    if (wb) ok = ok && tile_map(&M.co, fp32 ? op->pack32 : op->pack64, st, wb / 4, wb / 4, A.tx, A.ty);
+    if (!ok) return false;
+    TileStep<TM, TC> S;
+    S.y = (TM*)y;
+    S.sig = sig;
+    S.alpha = s_from<TC>(alpha, 0.0);
+    S.beta = s_from<TC>(beta, 0.0);
+    S.gamma = s_from<TC>(gamma, 0.0);
+    const TileResid Q = {};
+    if (st.kind == TK_CSR7) return tile_launch<TK_CSR7, TS, TC, TM, SRC, false>(ctx, A, M, S, Q, grid, smem);
+    if constexpr (!IsComplex<TC>::value)
+        if (st.kind == TK_STENCIL27) return tile_launch<TK_STENCIL27, TS, TC, TM, SRC, false>(ctx, A, M, S, Q, grid, smem);
+    return tile_launch<TK_STENCIL7, TS, TC, TM, SRC, false>(ctx, A, M, S, Q, grid, smem);
+}
+
+bool tile_step(rc_ctx* ctx, const rc_op* op, TileType type, int64_t ld, const void* x, const void* z, void* y, double alpha,
+               double beta, double gamma, const void* src, const float* sig) {
+    if (((uintptr_t)x | (uintptr_t)z | (uintptr_t)y | (uintptr_t)src) % 16) return false;
+    switch (type) {
+        case TT_F64:
+            return tile_step_t<double, double, double, false>(ctx, op, type, ld, x, z, y, alpha, beta, gamma, src, sig);
+        case TT_C128:
+            return tile_step_t<double2, double2, double2, false>(ctx, op, type, ld, x, z, y, alpha, beta, gamma, src, sig);
+        case TT_BF16:
+            return tile_step_t<float, float, __nv_bfloat16, true>(ctx, op, type, ld, x, z, y, alpha, beta, gamma, src, sig);
+        case TT_BF16C:
+            return tile_step_t<float2, float2, __nv_bfloat162, true>(ctx, op, type, ld, x, z, y, alpha, beta, gamma, src,
+                                                                     sig);
+    }
+    return false;
+}
+
+template <class T>
+static bool tile_resid_t(rc_ctx* ctx, const rc_op* op, const void* Y, int64_t ld, TileResid Q, int64_t res_count,
+                         double** part, int64_t* parts, rc_status* status) {
+    const Structure st = structure(op, false);
+    TileArgs A;
+    unsigned grid;
+    size_t smem;
+    const int wb = st.kind == TK_CSR7 ? (int)sizeof(RowWeights<T>) : 0;
+    const int64_t words = ld * (int64_t)sizeof(T) / 4;
+    if (!tile_plan(ctx, st, (int)(words / 4), 0, wb, &A, &grid, &smem)) return false;
+    A.ld = ld;
+    A.off = op->offdiag;
+    A.diag = op->diag64;
+    A.phase = op->phase64;
+    TileMaps M = {};
+    bool ok = tile_map(&M.x, Y, st, words, A.nseg * 4, A.tx + 2, A.ty + 2);
+    if (wb) ok = ok && tile_map(&M.co, op->pack64, st, wb / 4, wb / 4, A.tx, A.ty);
+    if (!ok) return false;
+    if (res_count > 0) {
+        void* p = nullptr;
+        *status = rc_slot(ctx, S_RPART, (size_t)grid * res_count * sizeof(double), &p);
+        if (*status != RC_OK) return true;
+        Q.part = *part = (double*)p;
+        *parts = grid;
+    }
+    const TileStep<T, T> S = {};
+    if (st.kind == TK_CSR7) return tile_launch<TK_CSR7, T, T, T, false, true>(ctx, A, M, S, Q, grid, smem);
+    if constexpr (!IsComplex<T>::value)
+        if (st.kind == TK_STENCIL27) return tile_launch<TK_STENCIL27, T, T, T, false, true>(ctx, A, M, S, Q, grid, smem);
+    return tile_launch<TK_STENCIL7, T, T, T, false, true>(ctx, A, M, S, Q, grid, smem);
+}
+
+bool tile_resid(rc_ctx* ctx, const rc_op* op, const void* Y, int64_t ld, int64_t s, const double* lam, int64_t res_count,
+                void* R, int64_t ldr, double** part, int64_t* parts, rc_status* st) {
+    *st = RC_OK;
+    if ((uintptr_t)Y % 16 || (uintptr_t)R % 4) return false;
+    TileResid Q = {};
+    Q.lam = lam;
+    Q.R = R;
+    Q.ldr = ldr;
+    Q.res_count = (int)res_count;
+    Q.s = s;
+    return op->dtype == RC_COMPLEX128 ? tile_resid_t<double2>(ctx, op, Y, ld, Q, res_count, part, parts, st)
+                                      : tile_resid_t<double>(ctx, op, Y, ld, Q, res_count, part, parts, st);
+}
+
+rc_status tile_pack(rc_ctx* ctx, const rc_op* op, bool fp32, const void* vals, void** out, size_t* bytes) {
+    const bool cplx = op->dtype == RC_COMPLEX128;
+    *bytes = (size_t)op->n * 8 * elem_bytes(op->dtype, fp32 ? P32 : P64);
+    if (cudaMalloc(out, *bytes) != cudaSuccess) {
+        cudaGetLastError();
+        *out = nullptr;
+        return rc_fail(ctx, RC_ERR_NOMEM, "cudaMalloc for operator storage failed");
+    }
+    const unsigned g = (unsigned)std::min<int64_t>((op->n + 255) / 256, 16 * kB200Sms);
+    const int nx = (int)op->gx, ny = (int)op->gy, nz = (int)op->gz;
+    if (cplx && fp32)
+        tile_pack_kernel<float2><<<g, 256, 0, ctx->stream>>>(op->n, nx, ny, nz, op->rowptr, (const float2*)vals,
+                                                             (RowWeights<float2>*)*out);
+    else if (cplx)
+        tile_pack_kernel<double2><<<g, 256, 0, ctx->stream>>>(op->n, nx, ny, nz, op->rowptr, (const double2*)vals,
+                                                              (RowWeights<double2>*)*out);
+    else if (fp32)
+        tile_pack_kernel<float><<<g, 256, 0, ctx->stream>>>(op->n, nx, ny, nz, op->rowptr, (const float*)vals,
+                                                            (RowWeights<float>*)*out);
+    else
+        tile_pack_kernel<double><<<g, 256, 0, ctx->stream>>>(op->n, nx, ny, nz, op->rowptr, (const double*)vals,
+                                                             (RowWeights<double>*)*out);
+    ctx->launches++;
+    RC_CU(ctx, cudaGetLastError());
+    return RC_OK;
+}
+
+}  // namespace rcb

@@ -1,0 +1,23 @@
+// rc_tile.h -- the shared-memory tile kernels of 7- and 27-point operators (rc_tile.cu).
+#pragma once
+#include "rc_internal.h"
+
+namespace rcb {
+
+// Storage of a step's blocks: FP64, c128, or the correction filter's bfloat16 (pairs) with FP32 (c64) arithmetic.
+enum TileType { TT_F64 = 0, TT_C128, TT_BF16, TT_BF16C };
+
+// Whether the operator has the structure and the block (row length ld) the size for the tile kernels.
+bool tile_supported(const rc_ctx* ctx, const rc_op* op, TileType type, int64_t ld);
+// y = alpha A x + beta x + gamma z (+ sig[c] src): rm_step_rows' step; z may be null, src goes with TT_BF16*.
+// False (nothing launched) when a pointer is not 16-byte aligned or the driver refuses a tensor map.
+bool tile_step(rc_ctx* ctx, const rc_op* op, TileType type, int64_t ld, const void* x, const void* z, void* y, double alpha,
+               double beta, double gamma, const void* src, const float* sig);
+// The residual block of rc_resid.cu (FP64 / c128 Y): R (or null) and the partial column sums of squares of *parts CTAs
+// into S_RPART.
+bool tile_resid(rc_ctx* ctx, const rc_op* op, const void* Y, int64_t ld, int64_t s, const double* lam, int64_t res_count,
+                void* R, int64_t ldr, double** part, int64_t* parts, rc_status* st);
+// Weights of CSR rows with the 7-point structure, in the tile kernels' order: from the operator's values.
+rc_status tile_pack(rc_ctx* ctx, const rc_op* op, bool fp32, const void* vals, void** out, size_t* bytes);
+
+}  // namespace rcb
