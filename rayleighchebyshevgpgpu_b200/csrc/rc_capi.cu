@@ -235,12 +235,15 @@ static rc_status dev_copy(rc_ctx* ctx, void** dst, const void* src, size_t bytes
     return RC_OK;
 }
 
-// Whether the rows are those of a 7-point stencil on a grid: offsets 0, +-1, +-L, +-P with L | P | n, and row i holds
-// the diagonal and exactly the neighbours that lie in the grid, columns ascending. Sets op->gx, gy, gz.
+// Whether the rows are those of a 7-point stencil on a grid of at least two points each way: row 0 holds the columns
+// 0, 1, L and P with L | P | n, and row i the diagonal and exactly the neighbours that lie in the grid, columns
+// ascending. Then it sets op->gx, gy, gz; every index is in range and the column offsets are 0, +-1, +-L and +-P.
+// It stops at the first row that differs. rowptr has been checked.
 static void csr_grid(rc_op* op, const int32_t* rowptr, const int32_t* colind) {
-    const int64_t* o = op->offsets;
-    const int64_t L = o[5], P = o[6], n = op->n;
-    if (o[3] != 0 || o[4] != 1 || o[2] != -1 || L < 2 || o[1] != -L || o[0] != -P || P <= L || P % L || n % P) return;
+    const int64_t n = op->n;
+    if (rowptr[1] != 4 || colind[0] != 0 || colind[1] != 1) return;
+    const int64_t L = colind[2], P = colind[3];
+    if (L < 2 || P <= L || P >= n || P % L || n % P) return;
     const int64_t ny = P / L, nz = n / P;
     int64_t i = 0;
     for (int64_t z = 0; z < nz; ++z)
@@ -278,27 +281,6 @@ rc_status rc_op_csr_create(rc_ctx* ctx, int dtype, int64_t n, int64_t nnz, const
         if (rowptr[i + 1] < rowptr[i]) return rc_fail(ctx, RC_ERR_INVALID, "rowptr not non-decreasing");
         max_row = std::max<int64_t>(max_row, rowptr[i + 1] - rowptr[i]);
     }
-    for (int64_t k = 0; k < nnz; ++k)
-        if (colind[k] < 0 || colind[k] >= n) return rc_fail(ctx, RC_ERR_INVALID, "column index out of range");
-    int64_t band = 0;
-    std::vector<int64_t> offs;  // distinct column offsets, while there are few
-    bool few = true;
-    size_t at = 0;  // where the last offset was found: the next one usually follows it
-    for (int64_t i = 0; i < n; ++i)
-        for (int32_t k = rowptr[i]; k < rowptr[i + 1]; ++k) {
-            const int64_t o = (int64_t)colind[k] - i;
-            band = std::max<int64_t>(band, o);
-            if (!few) continue;
-            if (at + 1 < offs.size() && offs[at + 1] == o) {
-                ++at;
-                continue;
-            }
-            at = (size_t)(std::find(offs.begin(), offs.end(), o) - offs.begin());
-            if (at == offs.size()) {
-                offs.push_back(o);
-                few = (int)offs.size() <= rc_op::kMaxOffsets;
-            }
-        }
     rc_op* op = new (std::nothrow) rc_op();
     if (!op) return RC_ERR_NOMEM;
     op->ctx = ctx;
@@ -307,13 +289,44 @@ rc_status rc_op_csr_create(rc_ctx* ctx, int dtype, int64_t n, int64_t nnz, const
     op->n = n;
     op->nnz = nnz;
     op->max_row_nnz = max_row;
-    op->band = band;
-    if (few) {
-        std::sort(offs.begin(), offs.end());
-        op->n_offsets = (int)offs.size();
-        for (size_t q = 0; q < offs.size(); ++q) op->offsets[q] = offs[q];
+    csr_grid(op, rowptr, colind);
+    if (op->gx > 0) {
+        const int64_t L = op->gx, P = L * op->gy;
+        const int64_t offs[7] = {-P, -L, -1, 0, 1, L, P};
+        op->band = P;
+        op->n_offsets = 7;
+        std::copy(offs, offs + 7, op->offsets);
+    } else {
+        uint32_t top = 0;  // a negative index is a large unsigned one
+        for (int64_t k = 0; k < nnz; ++k) top = std::max(top, (uint32_t)colind[k]);
+        if (nnz > 0 && (int64_t)top >= n) {
+            delete op;
+            return rc_fail(ctx, RC_ERR_INVALID, "column index out of range");
+        }
+        std::vector<int64_t> offs;  // distinct column offsets, while there are few
+        bool few = true;
+        size_t at = 0;  // where the last offset was found: the next one usually follows it
+        for (int64_t i = 0; i < n; ++i)
+            for (int32_t k = rowptr[i]; k < rowptr[i + 1]; ++k) {
+                const int64_t o = (int64_t)colind[k] - i;
+                op->band = std::max<int64_t>(op->band, o);
+                if (!few) continue;
+                if (at + 1 < offs.size() && offs[at + 1] == o) {
+                    ++at;
+                    continue;
+                }
+                at = (size_t)(std::find(offs.begin(), offs.end(), o) - offs.begin());
+                if (at == offs.size()) {
+                    offs.push_back(o);
+                    few = (int)offs.size() <= rc_op::kMaxOffsets;
+                }
+            }
+        if (few) {
+            std::sort(offs.begin(), offs.end());
+            op->n_offsets = (int)offs.size();
+            for (size_t q = 0; q < offs.size(); ++q) op->offsets[q] = offs[q];
+        }
     }
-    if (op->n_offsets == 7) csr_grid(op, rowptr, colind);
     const size_t vsz = (dtype == RC_COMPLEX128 ? 16 : 8);
     rc_status st = dev_copy(ctx, (void**)&op->rowptr, rowptr, (size_t)(n + 1) * 4, op);
     if (st == RC_OK) st = dev_copy(ctx, (void**)&op->colind, colind, (size_t)nnz * 4, op);
@@ -324,6 +337,9 @@ rc_status rc_op_csr_create(rc_ctx* ctx, int dtype, int64_t n, int64_t nnz, const
         if (st == RC_OK) {
             op->bytes += (int64_t)b;
             ctx->op_bytes += (int64_t)b;
+            // other contexts' streams may use the operator as soon as it exists (its other arrays are copied in order)
+            if (cudaStreamSynchronize(ctx->stream) != cudaSuccess)
+                st = rc_fail(ctx, RC_ERR_CUDA, "rc_op_csr_create: packing the weights failed");
         }
     }
     if (st != RC_OK) {

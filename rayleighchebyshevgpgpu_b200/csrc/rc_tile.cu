@@ -17,6 +17,10 @@
 // reads instead of 8 (27 points: 4.5 instead of 9), no address or bounds arithmetic per neighbour, and nothing
 // waits on DRAM but the producer. The sums are formed in the gather kernels' order (5- and 7-point: the same bits).
 //
+// Measured, against the gather kernels (time per step; HBM floor): CSR 128^3, 96 columns, bfloat16 347 -> 242 us (246),
+// FP64 1146 -> 758 (760); 27 points 192^3, 48 columns, bfloat16 992 -> 467 (415), FP64 residual block 2204 -> 1016;
+// complex stencil, 884,736 rows x 192 columns, bfloat16 pairs 570 -> 482 (415), bound by instruction issue.
+//
 // Units (a panel of a tile over ml planes) are taken in turn by one CTA per SM, panels fastest, then x, y, z: the
 // tiles in flight are neighbours, so a halo's rows are read from DRAM once. ml is chosen so that the last turn is
 // nearly full (tile_plan).
@@ -32,13 +36,17 @@ namespace rcb {
 
 namespace {
 
-// Smallest block (bytes) for which the tile kernels are taken.
-constexpr int64_t kTileMinBytes = 32ll << 20;
+// Smallest block (bytes) for which the tile kernels are taken for 7 points: below, both forms take a launch's latency
+// (24^3, 24 FP64 columns, 2.7 MB: 68 us for 5 steps either way; 24^3, 96 columns: 88 -> 73 us). 27 points: always
+// (8^3, 24 columns: 303 -> 69 us).
+constexpr int64_t kTileMinBytes = 4ll << 20;
 
 enum { TK_STENCIL7 = 0, TK_CSR7 = 1, TK_STENCIL27 = 2 };
-constexpr int TL_ROWS = 4;          // points along y per thread
+// Points along y per thread. 27 points: the sums of three planes of four points spill at 128 registers.
+constexpr int tl_rows(int kind) { return kind == TK_STENCIL27 ? 2 : 4; }
 constexpr int TL_MAX_SLOTS = 4;
 constexpr int TL_MAX_SEG = 12;      // slices per panel, at most
+constexpr int TL_MAX_SEG27 = 6;     // 27 points
 constexpr int TL_THREADS = 384;     // product threads, at most
 
 // What a kernel needs beside the maps. Sizes in bytes; slots are multiples of 128.
@@ -83,6 +91,13 @@ __device__ __forceinline__ void tma_load_4d(uint32_t dst, const CUtensorMap* map
         : "memory");
 }
 
+// A 16-byte shared-memory read, as one instruction (as two 8-byte ones, FP64 slices had two-way bank conflicts).
+__device__ __forceinline__ uint4 lds16(uint32_t a) {
+    uint4 u;
+    asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(u.x), "=r"(u.y), "=r"(u.z), "=r"(u.w) : "r"(a));
+    return u;
+}
+
 struct Unit {
     int panel, x0, y0, m0, m1;
 };
@@ -113,15 +128,34 @@ struct Ring {
 template <class TS, class TC, class TM>
 struct TileVec {
     static constexpr int V = Slice<TS, TM>::V;
-    // a += c x in the gather kernels' rounding (packed FP32 pairs for bfloat16 blocks)
+    // a += c x in the gather kernels' rounding (packed FP32 pairs for bfloat16 blocks and c64)
     __device__ static __forceinline__ void add(TC (&a)[V], TC c, const uint4& u) {
         const Slice<TS, TM> p = slice_from<TS, TM>(u);
         if constexpr (sizeof(TM) == 2) {
 #pragma unroll
             for (int v = 0; v < V; v += 2) ffma2(c, c, p.v[v], p.v[v + 1], a[v], a[v + 1]);
+        } else if constexpr (std::is_same<TC, float2>::value) {
+#pragma unroll
+            for (int v = 0; v < V; ++v) {
+                ffma2(-c.y, c.y, p.v[v].y, p.v[v].x, a[v].x, a[v].y);
+                ffma2(c.x, c.x, p.v[v].x, p.v[v].y, a[v].x, a[v].y);
+            }
         } else {
 #pragma unroll
             for (int v = 0; v < V; ++v) a[v] = s_fma(c, s_cvt<TC>(p.v[v]), a[v]);
+        }
+    }
+    // the same for a real c: the products with its zero imaginary part left out
+    __device__ static __forceinline__ void addr(TC (&a)[V], real_t<TC> c, const uint4& u) {
+        if constexpr (IsComplex<TC>::value) {
+            const Slice<TS, TM> p = slice_from<TS, TM>(u);
+#pragma unroll
+            for (int v = 0; v < V; ++v) {
+                if constexpr (sizeof(c) == 4) ffma2(c, c, p.v[v].x, p.v[v].y, a[v].x, a[v].y);
+                else a[v] = make_double2(fma(c, p.v[v].x, a[v].x), fma(c, p.v[v].y, a[v].y));
+            }
+        } else {
+            add(a, c, u);
         }
     }
 };
@@ -135,7 +169,7 @@ struct RowWeights {
 template <int KIND, class TS, class TC, class TM, bool SRC, bool RESID>
 __global__ void __launch_bounds__(TL_THREADS + 32, 1)
 tile_kernel(TileArgs A, const __grid_constant__ TileMaps M, TileStep<TM, TC> S, TileResid Q) {
-    constexpr int V = Slice<TS, TM>::V;
+    constexpr int V = Slice<TS, TM>::V, TL_ROWS = tl_rows(KIND);
     constexpr bool CPLX = IsComplex<TC>::value;
     using TD = real_t<TC>;
     using Vec = TileVec<TS, TC, TM>;
@@ -259,7 +293,7 @@ tile_kernel(TileArgs A, const __grid_constant__ TileMaps M, TileStep<TM, TC> S, 
         };
         fetch_diag(U.m0);
         // the finished sums a (A x, or the box sum) of point k of plane m, whose own value is xi
-        auto finish = [&](int m, int k, const TC (&a)[V], const uint4& xr, const unsigned char* zb) {
+        auto finish = [&](int m, int k, const TC (&a)[V], const uint4& xr, uint32_t zb) {
             const Slice<TS, TM> xi = slice_from<TS, TM>(xr);
             const int64_t i = i0 + (int64_t)k * A.nx + (int64_t)m * plane;
             if constexpr (RESID) {
@@ -287,8 +321,8 @@ tile_kernel(TileArgs A, const __grid_constant__ TileMaps M, TileStep<TM, TC> S, 
                 }
             } else {
                 Slice<TS, TM> zi{}, si{}, out;
-                if (A.has_z) zi = slice_from<TS, TM>(*reinterpret_cast<const uint4*>(zb + zo + k * zp));
-                if (SRC) si = slice_from<TS, TM>(*reinterpret_cast<const uint4*>(zb + (A.zops - 1) * A.zbytes + zo + k * zp));
+                if (A.has_z) zi = slice_from<TS, TM>(lds16(zb + zo + k * zp));
+                if (SRC) si = slice_from<TS, TM>(lds16(zb + (A.zops - 1) * A.zbytes + zo + k * zp));
                 if constexpr (sizeof(TM) == 2) {
 #pragma unroll
                     for (int v = 0; v < V; v += 2) {
@@ -324,18 +358,17 @@ tile_kernel(TileArgs A, const __grid_constant__ TileMaps M, TileStep<TM, TC> S, 
         };
         auto wait_x = [&]() {
             ok = ok && mbar_wait(xfull + 8 * rx.slot, rx.ph);
-            return xs0 + rx.slot * A.xbytes + xo;
+            return smem_u32(xs0) + rx.slot * A.xbytes + xo;
         };
         auto free_x = [&](int slot) {
             __syncwarp();
             if (lane == 0) mbar_arrive(xempty + 8 * slot);
         };
-        auto ld16 = [](const unsigned char* p) { return *reinterpret_cast<const uint4*>(p); };
-        const unsigned char* zb = nullptr;
+        uint32_t zb = 0;
         auto wait_z = [&]() {
             if (!zring) return;
             ok = ok && mbar_wait(zfull + 8 * rz.slot, rz.ph);
-            zb = zs0 + rz.slot * zslot;
+            zb = smem_u32(zs0) + rz.slot * zslot;
         };
         auto free_z = [&]() {
             if (!zring) return;
@@ -345,12 +378,12 @@ tile_kernel(TileArgs A, const __grid_constant__ TileMaps M, TileStep<TM, TC> S, 
         };
         if constexpr (KIND == TK_STENCIL27) {
             // 3x3 sums of the four points in one plane, and their own values
-            auto plane_sums = [&](const unsigned char* p, TC (&b)[TL_ROWS][V], uint4 (&own)[TL_ROWS]) {
+            auto plane_sums = [&](uint32_t p, TC (&b)[TL_ROWS][V], uint4 (&own)[TL_ROWS]) {
 #pragma unroll
                 for (int l = 0; l < TL_ROWS + 2; ++l) {
-                    const uint4 c = ld16(p + l * xp);
-                    const Slice<TS, TM> cl = slice_from<TS, TM>(ld16(p + l * xp - cb)), cc = slice_from<TS, TM>(c),
-                                        cr = slice_from<TS, TM>(ld16(p + l * xp + cb));
+                    const uint4 c = lds16(p + l * xp);
+                    const Slice<TS, TM> cl = slice_from<TS, TM>(lds16(p + l * xp - cb)), cc = slice_from<TS, TM>(c),
+                                        cr = slice_from<TS, TM>(lds16(p + l * xp + cb));
                     if (l >= 1 && l <= TL_ROWS) own[l - 1] = c;
                     TC t[V];
 #pragma unroll
@@ -409,13 +442,13 @@ tile_kernel(TileArgs A, const __grid_constant__ TileMaps M, TileStep<TM, TC> S, 
         } else {
             uint4 um[TL_ROWS];  // the points below
             {
-                const unsigned char* p = wait_x();
+                const uint32_t p = wait_x();
 #pragma unroll
-                for (int k = 0; k < TL_ROWS; ++k) um[k] = ld16(p + (k + 1) * xp);
+                for (int k = 0; k < TL_ROWS; ++k) um[k] = lds16(p + (k + 1) * xp);
                 free_x(rx.slot);
                 rx.next(A.xslots);
             }
-            const unsigned char* pc = wait_x();
+            uint32_t pc = wait_x();
             int sc = rx.slot;
             rx.next(A.xslots);
             for (int m = U.m0; m < U.m1 && ok; ++m) {
@@ -425,28 +458,35 @@ tile_kernel(TileArgs A, const __grid_constant__ TileMaps M, TileStep<TM, TC> S, 
                     for (int k = 0; k < TL_ROWS; ++k) d[k] = dn[k];
                     fetch_diag(m + 1);
                 }
-                const unsigned char* pn = wait_x();
+                const uint32_t pn = wait_x();
                 wait_z();
-                uint4 c0 = ld16(pc), c1 = ld16(pc + xp);
+                uint4 c0 = lds16(pc), c1 = lds16(pc + xp);
 #pragma unroll
                 for (int k = 0; k < TL_ROWS; ++k) {
-                    const uint4 c2 = ld16(pc + (k + 2) * xp);
-                    const uint4 cl = ld16(pc + (k + 1) * xp - cb), cr = ld16(pc + (k + 1) * xp + cb);
-                    const uint4 cn = ld16(pn + (k + 1) * xp);
+                    const uint4 c2 = lds16(pc + (k + 2) * xp);
+                    const uint4 cl = lds16(pc + (k + 1) * xp - cb), cr = lds16(pc + (k + 1) * xp + cb);
+                    const uint4 cn = lds16(pn + (k + 1) * xp);
                     TC a[V];
 #pragma unroll
                     for (int v = 0; v < V; ++v) a[v] = s_zero(TC());
                     if constexpr (KIND == TK_STENCIL7) {
-                        Vec::add(a, s_from<TC>((double)d[k], 0.0), c1);
-                        Vec::add(a, off, um[k]);
+                        const TD w = (TD)A.off;
+                        Vec::addr(a, d[k], c1);
+                        Vec::addr(a, w, um[k]);
                         Vec::add(a, wm, c0);
-                        Vec::add(a, off, cl);
-                        Vec::add(a, off, cr);
+                        Vec::addr(a, w, cl);
+                        Vec::addr(a, w, cr);
                         Vec::add(a, wp, c2);
-                        Vec::add(a, off, cn);
+                        Vec::addr(a, w, cn);
                     } else {
-                        const RowWeights<TC>& w = *reinterpret_cast<const RowWeights<TC>*>(
-                            zb + A.zops * A.zbytes + ((ly + k) * A.tx + lx) * sizeof(RowWeights<TC>));
+                        RowWeights<TC> w;
+                        {
+                            uint4 r[sizeof(RowWeights<TC>) / 16];
+                            const uint32_t wa = zb + A.zops * A.zbytes + ((ly + k) * A.tx + lx) * (int)sizeof(RowWeights<TC>);
+#pragma unroll
+                            for (int e = 0; e < (int)(sizeof(r) / 16); ++e) r[e] = lds16(wa + 16 * e);
+                            memcpy(&w, r, sizeof(w));
+                        }
                         Vec::add(a, w.w[0], um[k]);
                         Vec::add(a, w.w[1], c0);
                         Vec::add(a, w.w[2], cl);
@@ -546,21 +586,37 @@ bool tile_plan(const rc_ctx* ctx, const Structure& S, int slices, int zops, int 
     A.ny = (int)S.ny;
     A.nz = (int)S.nz;
     A.slices = slices;
-    A.panels = (slices + TL_MAX_SEG - 1) / TL_MAX_SEG;
+    const int seg_max = S.kind == TK_STENCIL27 ? TL_MAX_SEG27 : TL_MAX_SEG, R = tl_rows(S.kind);
+    A.panels = (slices + seg_max - 1) / seg_max;
     A.nseg = (slices + A.panels - 1) / A.panels;
-    A.tx = A.nseg > 3 ? 16 : 32;
-    A.ltx = A.nseg > 3 ? 4 : 5;
-    A.ty = A.nseg > 6 ? 8 : 16;
     A.zops = zops;
     auto up = [](int b) { return (b + 127) / 128 * 128; };
+    const int room = (int)ctx->smem_optin - 2048;
+    // The tile: whole warps of at most TL_THREADS, three slots of x; the least memory traffic over the grid, points of
+    // the tiles past its edges included. A halo point costs half (it is in L2), a plane about 24 points by itself.
+    double least = 1e300;
+    for (int ltx = 2; ltx <= 5; ++ltx)
+        for (int ty = R; ty <= 32; ty += R) {
+            const int tx = 1 << ltx, nt = tx * ty / R * A.nseg;
+            if (nt > TL_THREADS || nt % 32) continue;
+            const int xb = up(A.nseg * 16 * (tx + 2) * (ty + 2)), zb = zops * up(A.nseg * 16 * tx * ty) + up(wbytes * tx * ty);
+            if (3 * xb + (zb ? 2 : 0) * zb > room) continue;
+            const double tiles = (double)((A.nx + tx - 1) / tx) * ((A.ny + ty - 1) / ty);
+            const double cost = tiles * (tx * ty * (2.0 + zops) + 0.5 * ((tx + 2) * (ty + 2) - tx * ty) + 24.0);
+            if (cost < least) {
+                least = cost;
+                A.tx = tx;
+                A.ltx = ltx;
+                A.ty = ty;
+            }
+        }
+    if (!A.tx) return false;
     A.xbytes = up(A.nseg * 16 * (A.tx + 2) * (A.ty + 2));
     A.zbytes = up(A.nseg * 16 * A.tx * A.ty);
     A.cbytes = up(wbytes * A.tx * A.ty);
     const int zslot = zops * A.zbytes + A.cbytes;
-    const int room = (int)ctx->smem_optin - 2048;
     A.zslots = zslot ? 2 : 1;
     A.xslots = std::min(TL_MAX_SLOTS, (room - A.zslots * zslot) / A.xbytes);
-    if (A.xslots < 3) return false;
     if (zslot && A.xslots == TL_MAX_SLOTS && 3 * zslot + A.xslots * A.xbytes <= room) A.zslots = 3;
     A.ntx = (A.nx + A.tx - 1) / A.tx;
     A.nty = (A.ny + A.ty - 1) / A.ty;
@@ -584,7 +640,7 @@ bool tile_plan(const rc_ctx* ctx, const Structure& S, int slices, int zops, int 
     *grid = (unsigned)std::min<int64_t>(ctas, A.units);
     // a CTA keeps its panel: whole turns of the panels
     *grid = *grid / A.panels * A.panels;
-    const int red = A.tx * A.ty / TL_ROWS * A.nseg * 2 * 8;  // the residual's column sums
+    const int red = A.tx * A.ty / R * A.nseg * 2 * 8;  // the residual's column sums
     *smem = (size_t)std::max(A.xslots * A.xbytes + A.zslots * zslot, red);
     *out = A;
     return true;
@@ -604,7 +660,7 @@ bool tile_launch(rc_ctx* ctx, const TileArgs& A, const TileMaps& M, const TileSt
         cudaGetLastError();
         return false;
     }
-    const int nt = A.tx * A.ty / TL_ROWS * A.nseg;
+    const int nt = A.tx * A.ty / tl_rows(KIND) * A.nseg;
     kern<<<grid, nt + 32, smem, ctx->stream>>>(A, M, S, Q);
     ctx->launches++;
     return true;
@@ -617,7 +673,7 @@ bool tile_supported(const rc_ctx* ctx, const rc_op* op, TileType type, int64_t l
     const Structure S = structure(op, type == TT_BF16 || type == TT_BF16C);
     if (S.kind < 0 || (op->dtype == RC_COMPLEX128) != (type == TT_C128 || type == TT_BF16C)) return false;
     if (S.kind == TK_STENCIL27 && op->dtype == RC_COMPLEX128) return false;
-    return ctx->tile > 1 || op->n * ld * tile_elem(type) >= kTileMinBytes;
+    return ctx->tile > 1 || S.kind == TK_STENCIL27 || op->n * ld * tile_elem(type) >= kTileMinBytes;
 }
 
 template <class TS, class TC, class TM, bool SRC>
