@@ -592,11 +592,11 @@ rc_status rc_rayleigh_ritz(rc_ctx* ctx, const rc_op* op_c, void* V, void* W, int
     RC_TRY(rcb::gram(ctx, dt, n, s, s, V, ld, W, ld, H, true));
     RC_TRY(rcb::small_eigh(ctx, dt, s, H, Qd, dlam, dinfo));
     if (op->kind != 2) {
-        // native operators: V <- V Q (in place where one pass holds the columns), then W <- A V once more and
-        // the residual norms from the two blocks. Against W Q formed beside V Q by one SIMT kernel, and both
-        // blocks copied back: 6.3 instead of 11.2 ms on the 128^3 CSR operator with 96 columns, 12.3 instead of
-        // 23.9 ms on a complex 7-point stencil with 442,368 rows and 192 columns (a sparse product costs 1.2
-        // and 0.9 ms there, a second dense one 1.2 and 3.8 ms).
+        // native operators: V <- V Q (in place where one pass holds the columns), then W <- A V once more with the
+        // residual norms beside it, against W Q formed beside V Q by one SIMT kernel and both blocks copied back:
+        // 4.2 instead of 11.2 ms on the 128^3 CSR operator with 96 columns, 8.9 instead of 24.0 ms on a complex
+        // 7-point stencil with 442,368 rows and 192 columns (a sparse product costs 0.6 and 0.45 ms there, a second
+        // dense one 1.2 and 3.8 ms).
         if (rcb::xt_dmma_in_place(s)) {
             RC_TRY(rcb::xt_dmma(ctx, dt, n, s, s, V, ld, false, Qd, s, V, ld));
         } else {
@@ -605,8 +605,7 @@ rc_status rc_rayleigh_ritz(rc_ctx* ctx, const rc_op* op_c, void* V, void* W, int
             RC_TRY(rcb::xt_dmma(ctx, dt, n, s, s, V, ld, false, Qd, s, T1, n));
             RC_TRY(rcb::copy_cols(ctx, dt, T1, n, V, ld, n, s));
         }
-        RC_TRY(rcb::op_step(ctx, op, st));
-        RC_TRY(rcb::resid_norms(ctx, dt, n, res_count, V, ld, W, ld, dlam, dres));
+        RC_TRY(rcb::op_step_norms(ctx, op, st, res_count, dlam, dres));
     } else {
         void *T1 = nullptr, *T2 = nullptr;
         RC_TRY(rc_slot(ctx, S_T1, (size_t)n * s * esz, &T1));

@@ -69,6 +69,11 @@ RC_HD double s_abs2(double a) { return a * a; }
 RC_HD float s_abs2(float a) { return a * a; }
 RC_HD double s_abs2(double2 a) { return a.x * a.x + a.y * a.y; }
 RC_HD float s_abs2(float2 a) { return a.x * a.x + a.y * a.y; }
+// acc - lm y: a residual from A y.
+__device__ __forceinline__ double resid_sub(double lm, double y, double acc) { return fma(-lm, y, acc); }
+__device__ __forceinline__ double2 resid_sub(double lm, double2 y, double2 acc) {
+    return make_double2(fma(-lm, y.x, acc.x), fma(-lm, y.y, acc.y));
+}
 RC_HD double s_real(double a) { return a; }
 RC_HD double s_real(double2 a) { return a.x; }
 RC_HD double s_imag(double) { return 0.0; }

@@ -62,6 +62,14 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map
         ::"r"(dst), "l"(map), "r"(x), "r"(y), "r"(bar)
         : "memory");
 }
+__device__ __forceinline__ void tma_load_4d(uint32_t dst, const CUtensorMap* map, int c, int x, int y, int z,
+                                            uint32_t bar) {
+    asm volatile(
+        "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], "
+        "[%6];" ::"r"(dst),
+        "l"(map), "r"(c), "r"(x), "r"(y), "r"(z), "r"(bar)
+        : "memory");
+}
 // Wait for the phase of the given parity. Bounded (each try suspends for a while by itself): false when the
 // limit ran out, which only a lost copy could cause.
 constexpr int kMbarTries = 1 << 22;
@@ -108,8 +116,10 @@ inline bool tma_map_2d(CUtensorMap* map, const double* p, int64_t inner, int64_t
               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-// A tensor map of dense 4-D blocks of 32-bit words, dims[0] of them a multiple of 4 (what lies outside reads as zero).
-inline bool tma_map_words_4d(CUtensorMap* map, const void* p, const int64_t (&dims)[4], const int (&box)[4]) {
+// A tensor map of 4-D blocks of 32-bit words, dims[0] of them a multiple of 4 (what lies outside reads as zero): dense,
+// or the last dimension `outer` words apart.
+inline bool tma_map_words_4d(CUtensorMap* map, const void* p, const int64_t (&dims)[4], const int (&box)[4],
+                             int64_t outer = 0) {
     const TensorMapEncodeFn fn = tensor_map_encode();
     if (!fn) return false;
     cuuint64_t d[4], st[3];
@@ -119,6 +129,7 @@ inline bool tma_map_words_4d(CUtensorMap* map, const void* p, const int64_t (&di
         b[k] = (cuuint32_t)box[k];
         if (k < 3) st[k] = (k ? st[k - 1] : 4) * d[k];
     }
+    if (outer) st[2] = (cuuint64_t)outer * 4;
     return fn(map, CU_TENSOR_MAP_DATA_TYPE_INT32, 4, const_cast<void*>(p), d, st, b, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
               CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) ==
            CUDA_SUCCESS;

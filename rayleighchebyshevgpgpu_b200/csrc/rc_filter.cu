@@ -423,6 +423,9 @@ rc_status op_step(rc_ctx* ctx, rc_op* op, const StepArgs& a) {
         return RC_OK;
     }
     if (a.cp == P32) RC_TRY(ensure_fp32(ctx, op));
+    bool done = false;
+    RC_TRY(cm_step(ctx, op, a, nullptr, 0, nullptr, nullptr, &done));
+    if (done) return RC_OK;
     if (op->kind == 1 && op->skind == 27 && cplx)
         return rc_fail(ctx, RC_ERR_UNSUPPORTED, "27-point stencil is real only");
     if (cplx) return a.cp == P64 ? launch_step_c<true, P64>(ctx, op, a) : launch_step_c<true, P32>(ctx, op, a);

@@ -328,6 +328,8 @@ rc_status xt_dmma(rc_ctx* ctx, int dtype, int64_t n, int64_t k, int64_t nc, cons
                   double* Yrm = nullptr, int64_t ldyr = 0);
 
 // res[c] = ||W_c - lam_c V_c|| for c < res_count (device), column-major blocks (rc_resid.cu).
+// op_step, and into res the norms of y - lam x of the first res_count columns (one kernel where the tiles take it).
+rc_status op_step_norms(rc_ctx* ctx, rc_op* op, const StepArgs& st, int64_t res_count, const double* lam, double* res);
 rc_status resid_norms(rc_ctx* ctx, int dtype, int64_t n, int64_t res_count, const void* V, int64_t ldv, const void* W,
                       int64_t ldw, const double* lam, double* res);
 

@@ -40,11 +40,6 @@ __device__ __forceinline__ void corr_store2(void* p, float a, float b) {
 #endif
 #endif
 }
-__device__ __forceinline__ double resid_sub(double lm, double y, double acc) { return fma(-lm, y, acc); }
-__device__ __forceinline__ double2 resid_sub(double lm, double2 y, double2 acc) {
-    return make_double2(fma(-lm, y.x, acc.x), fma(-lm, y.y, acc.y));
-}
-
 // The 27-point form (real): each thread walks kRun27 consecutive rows and keeps the 3x3
 // cross-section sums of rows i-1, i and i+1 (rm_step_rows27's scheme), so a row gathers 9
 // neighbours instead of 27: (A y)_i = (diag_i - offd) y_i + offd (Q(i-1) + Q(i) + Q(i+1)).
@@ -264,6 +259,22 @@ rc_status resid_norms(rc_ctx* ctx, int dtype, int64_t n, int64_t res_count, cons
     RC_CU(ctx, cudaGetLastError());
     resid_norm_reduce_kernel<<<(unsigned)res_count, 256, 0, ctx->stream>>>(chunks, (int)res_count, (const double*)part,
                                                                            res);
+    ctx->launches++;
+    RC_CU(ctx, cudaGetLastError());
+    return RC_OK;
+}
+
+rc_status op_step_norms(rc_ctx* ctx, rc_op* op, const StepArgs& st, int64_t res_count, const double* lam, double* res) {
+    double* part = nullptr;
+    int64_t parts = 0;
+    bool done = false;
+    if (st.cp == P64) RC_TRY(cm_step(ctx, op, st, lam, res_count, &part, &parts, &done));
+    if (!done) {
+        RC_TRY(op_step(ctx, op, st));
+        return resid_norms(ctx, op->dtype, op->n, res_count, st.x, st.ldx, st.y, st.ldy, lam, res);
+    }
+    if (res_count < 1) return RC_OK;
+    resid_norm_reduce_kernel<<<(unsigned)res_count, 256, 0, ctx->stream>>>(parts, (int)res_count, part, res);
     ctx->launches++;
     RC_CU(ctx, cudaGetLastError());
     return RC_OK;

@@ -82,15 +82,6 @@ struct TileMaps {
     CUtensorMap x, z, src, co;
 };
 
-__device__ __forceinline__ void tma_load_4d(uint32_t dst, const CUtensorMap* map, int c, int x, int y, int z,
-                                            uint32_t bar) {
-    asm volatile(
-        "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], "
-        "[%6];" ::"r"(dst),
-        "l"(map), "r"(c), "r"(x), "r"(y), "r"(z), "r"(bar)
-        : "memory");
-}
-
 // A 16-byte shared-memory read, as one instruction (as two 8-byte ones, FP64 slices had two-way bank conflicts).
 __device__ __forceinline__ uint4 lds16(uint32_t a) {
     uint4 u;
@@ -158,12 +149,6 @@ struct TileVec {
             add(a, c, u);
         }
     }
-};
-
-// One row of weights in shared memory: -P, -L, -1, 0, 1, L, P, (unused).
-template <class TC>
-struct RowWeights {
-    TC w[8];
 };
 
 template <int KIND, class TS, class TC, class TM, bool SRC, bool RESID>

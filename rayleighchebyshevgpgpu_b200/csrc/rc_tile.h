@@ -17,7 +17,17 @@ bool tile_step(rc_ctx* ctx, const rc_op* op, TileType type, int64_t ld, const vo
 // into S_RPART.
 bool tile_resid(rc_ctx* ctx, const rc_op* op, const void* Y, int64_t ld, int64_t s, const double* lam, int64_t res_count,
                 void* R, int64_t ldr, double** part, int64_t* parts, rc_status* st);
+// One row of packed weights: the neighbours at -P, -L, -1, 0, 1, L, P, (unused).
+template <class TC>
+struct RowWeights {
+    TC w[8];
+};
 // Weights of CSR rows with the 7-point structure, in the tile kernels' order: from the operator's values.
 rc_status tile_pack(rc_ctx* ctx, const rc_op* op, bool fp32, const void* vals, void** out, size_t* bytes);
+// op_step of a column-major FP64 block from tiles in shared memory (rc_cmstep.cu): *done is false (nothing launched)
+// where the operator, the types or the size are not for it. res_count > 0: also the partial column sums of
+// |y - lam x|^2 of *parts tiles, in S_RPART.
+rc_status cm_step(rc_ctx* ctx, const rc_op* op, const StepArgs& a, const double* lam, int64_t res_count, double** part,
+                  int64_t* parts, bool* done);
 
 }  // namespace rcb
