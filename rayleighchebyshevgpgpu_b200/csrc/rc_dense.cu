@@ -288,7 +288,7 @@ rc_status xt(rc_ctx* ctx, int dtype, const XtArgs& a) {
     if (a.n <= 0 || a.nc <= 0) return RC_OK;
     if (a.X2 == nullptr)
         return xt_dmma(ctx, dtype, a.n, a.k, a.nc, a.X, a.ldx, false, a.T, a.ldt, a.Y, a.ldy, a.alpha, a.beta, a.Yrm,
-                       a.ldyr);
+                       a.ldyr, a.tri);
     // real fast path: residual-only dual products
     const bool res_only = a.Y2 == nullptr && a.lam != nullptr && (a.res_count > 0 || a.R32 != nullptr);
     if (a.alpha == 1.0 && a.beta == 0.0 && res_only && xt2_supported(dtype, a.k, a.nc))
@@ -1232,6 +1232,7 @@ rc_status cholqr(rc_ctx* ctx, int dtype, void* V, int64_t ld, int64_t n, int64_t
         xa.X = cur; xa.ldx = ldc;
         xa.T = Tm; xa.ldt = s;
         xa.Y = oth; xa.ldy = ldo;
+        xa.tri = true;
         RC_TRY(xt(ctx, dtype, xa));
         ++np;
         // read the flags of this pass

@@ -303,6 +303,7 @@ struct XtArgs {
     // optional: the residual block X2 T - Y diag(lam) (all nc columns) in row-major FP32 with
     // leading dimension ldr (real blocks with k, nc <= 96 only)
     float* R32 = nullptr; int64_t ldr = 0;
+    bool tri = false;  // T is upper triangular (plain products)
     // optional: a row-major FP64 copy of Y (plain products, real blocks)
     double* Yrm = nullptr; int64_t ldyr = 0;
 };
@@ -325,7 +326,7 @@ rc_status xt2(rc_ctx* ctx, int64_t n, int64_t k, int64_t nc, const double* X, in
 bool xt_dmma_in_place(int64_t nc);
 rc_status xt_dmma(rc_ctx* ctx, int dtype, int64_t n, int64_t k, int64_t nc, const void* X, int64_t ldx, bool x_rm,
                   const void* T, int64_t ldt, void* Y, int64_t ldy, double alpha = 1.0, double beta = 0.0,
-                  double* Yrm = nullptr, int64_t ldyr = 0);
+                  double* Yrm = nullptr, int64_t ldyr = 0, bool tri = false);
 
 // res[c] = ||W_c - lam_c V_c|| for c < res_count (device), column-major blocks (rc_resid.cu).
 // op_step, and into res the norms of y - lam x of the first res_count columns (one kernel where the tiles take it).

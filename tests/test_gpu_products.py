@@ -74,3 +74,19 @@ def test_gram_tiles(ctx, complex_, s, n, pad, shift):
     q, r = np.linalg.qr(V.T)
     ph = np.diag(r) / np.abs(np.diag(r))
     np.testing.assert_allclose(out[:, :n], (q * ph).T, rtol=0, atol=1e-13)
+
+
+@pytest.mark.parametrize("complex_", [False, True])
+@pytest.mark.parametrize("s,n,pad", [(193, 1500, 0), (217, 1501, 0), (385, 2000, 1)])
+def test_triangular_products_in_several_passes(ctx, complex_, s, n, pad):
+    """Products with an upper triangular T of more than 192 columns: a pass's first tiles end far down in T."""
+    import torch
+    rng = np.random.default_rng(s)
+    V = rng.standard_normal((s, n)) + (1j * rng.standard_normal((s, n)) if complex_ else 0)
+    Vd = torch.zeros((s, n + pad), dtype=torch.complex128 if complex_ else torch.float64, device="cuda")
+    Vd[:, :n] = torch.from_numpy(V)
+    torch.cuda.synchronize()
+    R.cholqr(ctx, Vd, n, s, complex_, ld=n + pad)
+    q, r = np.linalg.qr(V.T)
+    ph = np.diag(r) / np.abs(np.diag(r))
+    np.testing.assert_allclose(Vd.cpu().numpy()[:, :n], (q * ph).T, rtol=0, atol=1e-13)
