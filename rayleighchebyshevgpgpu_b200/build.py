@@ -21,7 +21,7 @@ NVCC_FLAGS = ARCH_FLAGS + [
     "-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "-Xcompiler", "-O3",
     "--expt-relaxed-constexpr", "-Xptxas", "-O3",
 ]
-SOURCES = ["rc_filter.cu", "rc_filter_rm.cu", "rc_dense.cu", "rc_gemm.cu", "rc_xt.cu", "rc_tile.cu", "rc_cmstep.cu", "rc_gram.cu", "rc_jacobi.cu", "rc_noalloc.cu", "rc_lanczos.cu", "rc_solver.cu", "rc_capi.cu",
+SOURCES = ["rc_filter.cu", "rc_filter_rm.cu", "rc_dense.cu", "rc_gemm.cu", "rc_xt.cu", "rc_tile.cu", "rc_cmstep.cu", "rc_gram.cu", "rc_jacobi.cu", "rc_chol.cu", "rc_noalloc.cu", "rc_lanczos.cu", "rc_solver.cu", "rc_capi.cu",
            "rc_batch.cu", "rc_serve.cu", "rc_resid.cu", "rc_corrapi.cu"]
 
 

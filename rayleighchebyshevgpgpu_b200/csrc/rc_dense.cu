@@ -303,26 +303,19 @@ rc_status xt(rc_ctx* ctx, int dtype, const XtArgs& a) {
 // Cholesky factor of the column-scaled Gram matrix (one CTA, 1024 threads).
 //   d_i = sqrt(G_ii), Gh = D^-1 G D^-1 (+ sigma I on breakdown), Gh = R^H R (R upper),
 //   Tout = D^-1 R^-1 so that V*Tout has orthonormal columns.
-// The factor M and the inverse X live in dynamic shared memory when they fit (mode 2: both,
-// mode 1: M only), otherwise in global scratch that stays L2-resident. The inverse is formed
+// For more than 192 columns (up to there rc_chol.cu): the factor M and the inverse X live in global memory and stay
+// L2-resident. The inverse is formed
 // row by row from the bottom (X[i,j] for all j >= i in parallel), so no thread walks a long
 // dependent chain.
 // flags[0] |= 1 if shifted, flags[1] = 1 if failed, flags[2] = 1 if a zero column was met.
 template <class T>
 __global__ void __launch_bounds__(1024)
-chol_factor_kernel(int s, int64_t nrows, const T* __restrict__ G, T* Mg, T* Tout, double* dscg, int* flags, double* pivout,
-                   int mode) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
+chol_factor_kernel(int s, int64_t nrows, const T* __restrict__ G, T* M, T* Tout, double* dsc, int* flags,
+                   double* pivout) {
     __shared__ int s_bad;
     __shared__ double s_minpiv;
-    // In shared memory the matrices have an odd leading dimension (s + 1), so that a warp reading
-    // along a row (consecutive columns) hits distinct banks. The block is 32 x (blockDim/32):
-    // lane tx walks rows, warp ty walks columns, so no index needs a division.
-    const int lm = mode >= 1 ? s + 1 : s;
-    const int lx = mode == 2 ? s + 1 : s;
-    T* M = mode >= 1 ? (T*)smem_raw : Mg;
-    T* X = mode == 2 ? M + (size_t)s * lm : Tout;
-    double* dsc = mode == 2 ? (double*)(X + (size_t)s * lx) : (mode == 1 ? (double*)(M + (size_t)s * lm) : dscg);
+    // The block is 32 x (blockDim/32): lane tx walks rows, warp ty walks columns, so no index needs a division.
+    T* X = Tout;
     const int tid = threadIdx.x, nt = blockDim.x;
     const int tx = tid & 31, ty = tid >> 5, nwy = nt >> 5;
     for (int i = tid; i < s; i += nt) {
@@ -348,7 +341,7 @@ chol_factor_kernel(int s, int64_t nrows, const T* __restrict__ G, T* Mg, T* Tout
                 if (!isfinite(s_real(g)) || !isfinite(s_imag(g))) g = s_zero(T());
                 g = s_rscale(1.0 / (dsc[i] * dsc[j]), g);
                 if (i == j) g = s_from<T>(s_real(g) + shift, 0.0);
-                M[i + (int64_t)j * lm] = g;
+                M[i + (int64_t)j * s] = g;
             }
         __syncthreads();
         // right-looking upper Cholesky with one barrier per step: row k is final once step k-1
@@ -357,15 +350,15 @@ chol_factor_kernel(int s, int64_t nrows, const T* __restrict__ G, T* Mg, T* Tout
         // by sqrt(p_k) after the loop.
         bool bad = false;
         for (int k = 0; k < s; ++k) {
-            const double p = s_real(M[k + (int64_t)k * lm]);
+            const double p = s_real(M[k + (int64_t)k * s]);
             if (!(p > 1e-13)) bad = true;
             if (tid == 0) s_minpiv = fmin(s_minpiv, p);
             if (bad && attempt == 0) break;
             const double pinv = 1.0 / (p > 1e-300 ? p : 1e-300);
             for (int j = k + 1 + ty; j < s; j += nwy) {
-                const T mkj = s_rscale(pinv, M[k + (int64_t)j * lm]);
+                const T mkj = s_rscale(pinv, M[k + (int64_t)j * s]);
                 for (int i = k + 1 + tx; i <= j; i += 32)
-                    M[i + (int64_t)j * lm] = s_sub(M[i + (int64_t)j * lm], s_mul(s_conj(M[k + (int64_t)i * lm]), mkj));
+                    M[i + (int64_t)j * s] = s_sub(M[i + (int64_t)j * s], s_mul(s_conj(M[k + (int64_t)i * s]), mkj));
             }
             __syncthreads();
         }
@@ -385,29 +378,29 @@ chol_factor_kernel(int s, int64_t nrows, const T* __restrict__ G, T* Mg, T* Tout
     __syncthreads();
     // R[k,j] = M[k,j] / sqrt(p_k) (j > k), R[k,k] = sqrt(p_k); the pivots go through X first
     for (int k = tid; k < s; k += nt) {
-        const double p = s_real(M[k + (int64_t)k * lm]);
+        const double p = s_real(M[k + (int64_t)k * s]);
         X[k] = s_from<T>(sqrt(p > 1e-300 ? p : 1e-300), 0.0);
     }
     __syncthreads();
     for (int j = ty; j < s; j += nwy)
         for (int i = tx; i <= j; i += 32) {
             const double rkk = s_real(X[i]);
-            if (j > i) M[i + (int64_t)j * lm] = s_rscale(1.0 / rkk, M[i + (int64_t)j * lm]);
-            else M[i + (int64_t)i * lm] = s_from<T>(rkk, 0.0);
+            if (j > i) M[i + (int64_t)j * s] = s_rscale(1.0 / rkk, M[i + (int64_t)j * s]);
+            else M[i + (int64_t)i * s] = s_from<T>(rkk, 0.0);
         }
     __syncthreads();
     // X = R^-1 (upper), right-looking back substitution on all columns at once with one barrier
     // per step: Y starts as I; at step k (s-1 .. 1) row k of Y is final, and R[l,k] Y[k,:]/R[k,k]
     // is removed from the rows l < k. X[k,:] = Y[k,:]/R[k,k] is applied in the last pass.
     for (int j = ty; j < s; j += nwy)
-        for (int i = tx; i < s; i += 32) X[i + (int64_t)j * lx] = s_from<T>(i == j ? 1.0 : 0.0, 0.0);
+        for (int i = tx; i < s; i += 32) X[i + (int64_t)j * s] = s_from<T>(i == j ? 1.0 : 0.0, 0.0);
     __syncthreads();
     for (int k = s - 1; k >= 1; --k) {
-        const double inv = 1.0 / s_real(M[k + (int64_t)k * lm]);
+        const double inv = 1.0 / s_real(M[k + (int64_t)k * s]);
         for (int j = k + ty; j < s; j += nwy) {
-            const T ykj = s_rscale(inv, X[k + (int64_t)j * lx]);
+            const T ykj = s_rscale(inv, X[k + (int64_t)j * s]);
             for (int l = tx; l < k; l += 32)
-                X[l + (int64_t)j * lx] = s_sub(X[l + (int64_t)j * lx], s_mul(M[l + (int64_t)k * lm], ykj));
+                X[l + (int64_t)j * s] = s_sub(X[l + (int64_t)j * s], s_mul(M[l + (int64_t)k * s], ykj));
         }
         __syncthreads();
     }
@@ -415,37 +408,23 @@ chol_factor_kernel(int s, int64_t nrows, const T* __restrict__ G, T* Mg, T* Tout
     // Tout = D^-1 X = D^-1 diag(R)^-1 Y
     for (int j = ty; j < s; j += nwy)
         for (int i = tx; i < s; i += 32)
-            Tout[i + (int64_t)j * s] = s_rscale(1.0 / (dsc[i] * s_real(M[i + (int64_t)i * lm])), X[i + (int64_t)j * lx]);
+            Tout[i + (int64_t)j * s] = s_rscale(1.0 / (dsc[i] * s_real(M[i + (int64_t)i * s])), X[i + (int64_t)j * s]);
 }
 
 rc_status chol_factor(rc_ctx* ctx, int dtype, int64_t s, int64_t nrows, const void* G, void* Tout, int* flags,
                       double* pivout) {
+    rc_status st = RC_OK;
+    if (chol_registers(ctx, dtype, s, nrows, G, Tout, flags, pivout, &st)) return st;
     const size_t esz = dtype == RC_COMPLEX128 ? 16 : 8;
     void* base = nullptr;
     RC_TRY(rc_slot(ctx, S_LANCZOS, (size_t)s * s * esz + (size_t)s * 8 + 256, &base));
     double* dsc = (double*)((char*)base + (size_t)s * s * esz);
-    const size_t budget = ctx->smem_optin > 4096 ? ctx->smem_optin - 4096 : 0;
-    const size_t mat = (size_t)s * (s + 1) * esz;  // with the padded leading dimension
-    int mode = 0;
-    size_t dyn = 0;
-    if (2 * mat + (size_t)s * 8 <= budget) {
-        mode = 2;
-        dyn = 2 * mat + (size_t)s * 8;
-    } else if (mat + (size_t)s * 8 <= budget) {
-        mode = 1;
-        dyn = mat + (size_t)s * 8;
-    }
-    if (dtype == RC_COMPLEX128) {
-        if (dyn > 48 * 1024)
-            RC_CU(ctx, allow_max_smem(ctx, chol_factor_kernel<double2>));
-        chol_factor_kernel<double2><<<1, 1024, dyn, ctx->stream>>>((int)s, nrows, (const double2*)G, (double2*)base,
-                                                                  (double2*)Tout, dsc, flags, pivout, mode);
-    } else {
-        if (dyn > 48 * 1024)
-            RC_CU(ctx, allow_max_smem(ctx, chol_factor_kernel<double>));
-        chol_factor_kernel<double><<<1, 1024, dyn, ctx->stream>>>((int)s, nrows, (const double*)G, (double*)base,
-                                                                 (double*)Tout, dsc, flags, pivout, mode);
-    }
+    if (dtype == RC_COMPLEX128)
+        chol_factor_kernel<double2><<<1, 1024, 0, ctx->stream>>>((int)s, nrows, (const double2*)G, (double2*)base,
+                                                                (double2*)Tout, dsc, flags, pivout);
+    else
+        chol_factor_kernel<double><<<1, 1024, 0, ctx->stream>>>((int)s, nrows, (const double*)G, (double*)base,
+                                                               (double*)Tout, dsc, flags, pivout);
     ctx->launches++;
     RC_CU(ctx, cudaGetLastError());
     return RC_OK;

@@ -348,7 +348,10 @@ rc_status resid_block(rc_ctx* ctx, const rc_op* op, const void* Yrm, int64_t ld,
 // pivout (device, optional): smallest pivot of the scaled Cholesky (1 = orthonormal columns).
 rc_status chol_factor(rc_ctx* ctx, int dtype, int64_t s, int64_t nrows, const void* G, void* Tout,
                       int* flags, double* pivout);
-// Hermitian eigensolve (parallel Jacobi, one CTA). A (s x s) is read only; evals ascending.
+// Its form for up to 192 columns, in registers (rc_chol.cu): false (nothing launched) for more.
+bool chol_registers(rc_ctx* ctx, int dtype, int64_t s, int64_t nrows, const void* G, void* Tout, int* flags,
+                    double* pivout, rc_status* st);
+// Hermitian eigensolve (parallel Jacobi). A (s x s) is read only; evals ascending.
 rc_status small_eigh(rc_ctx* ctx, int dtype, int64_t s, void* A, void* Q, double* evals, int* info);
 // Same with caller-provided work memory (small_eigh_work_bytes(...) bytes, 0 when the working
 // copies fit in shared memory; 256-byte aligned).

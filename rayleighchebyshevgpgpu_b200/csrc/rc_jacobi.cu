@@ -30,6 +30,7 @@
 // sgn(d) 2 r w a_pq. The matrix is first scaled by a power of two to entries of at most 1 (exact), so that the
 // squares neither overflow nor underflow.
 #include <algorithm>
+#include "rc_cluster.cuh"
 #include "rc_common.cuh"
 #include "rc_internal.h"
 
@@ -37,37 +38,12 @@ namespace rcb {
 
 namespace {
 
-__device__ __forceinline__ unsigned jc_rank() {
-    unsigned r;
-    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-    return r;
-}
 // The same shared-memory location in CTA `rank` of the cluster, as a generic address.
 template <class U>
 __device__ __forceinline__ U* jc_at(U* p, unsigned rank) {
     unsigned long long a = (unsigned long long)p, o;
     asm("mapa.u64 %0, %1, %2;" : "=l"(o) : "l"(a), "r"(rank));
     return (U*)o;
-}
-template <bool CL>
-__device__ __forceinline__ void jc_sync() {
-    if constexpr (CL) {
-        asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-    } else {
-        __syncthreads();
-    }
-}
-// The shared::cluster address of `p` in CTA `rank`, and stores to such addresses.
-__device__ __forceinline__ uint32_t jc_addr(const void* p, unsigned rank) {
-    uint32_t o;
-    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(o) : "r"((uint32_t)__cvta_generic_to_shared(p)), "r"(rank));
-    return o;
-}
-__device__ __forceinline__ void jc_store(uint32_t a, double v) {
-    asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(a), "d"(v) : "memory");
-}
-__device__ __forceinline__ void jc_store(uint32_t a, double2 v) {
-    asm volatile("st.shared::cluster.v2.f64 [%0], {%1, %2};" ::"r"(a), "d"(v.x), "d"(v.y) : "memory");
 }
 // c x - conj(t) y and t x + c y
 __device__ __forceinline__ double jc_lo(double c, double t, double x, double y) { return fma(c, x, -t * y); }
@@ -121,7 +97,7 @@ jacobi_cluster_kernel(int s, int P, int C, const T* __restrict__ Ain, T* __restr
     extern __shared__ __align__(16) unsigned char jcs[];
     __shared__ double sc[32];
     const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31, warp = tid >> 5, nw = nt >> 5;
-    const int rank = CL ? (int)jc_rank() : 0;
+    const int rank = CL ? (int)cl_rank() : 0;
     const int np = P * C, sp = 2 * np, M = sp - 1, S = P + 1;
     const int csz = 2 * sp;                  // a column: sp rows of A, then sp rows of Q
     T* tops = (T*)jcs;
@@ -146,16 +122,16 @@ jacobi_cluster_kernel(int s, int P, int C, const T* __restrict__ Ain, T* __restr
     auto own_col = [&](int f) { return f < P ? top_at(th, f) : bot_at(bh, f - P); };
     // a value of this CTA to every CTA's ex[rank]
     auto share = [&](double v) {
-        jc_sync<CL>();
+        cl_sync<CL>();
         if (tid < C) (CL ? jc_at(ex, tid) : ex)[rank] = v;
-        jc_sync<CL>();
+        cl_sync<CL>();
     };
     auto share_diag = [&]() {
         for (int e = tid; e < 2 * P * C; e += nt) {
             const int k = e / (2 * P), f = e - k * 2 * P, x = own_index(f);
             (CL ? jc_at(diag, k) : diag)[x] = s_real(own_col(f)[x]);
         }
-        jc_sync<CL>();
+        cl_sync<CL>();
     };
 
     // the columns of round 0, a warp per column
@@ -204,11 +180,11 @@ jacobi_cluster_kernel(int s, int P, int C, const T* __restrict__ Ain, T* __restr
     // where the columns that leave go, with the heads at t0 and b0: the free slots of the neighbours (at the
     // ends of the cluster, of the own other row)
     auto leave_top = [&](int t0, int b0) {
-        return rank == 0 ? jc_addr(bots + b0 * csz, 0) : jc_addr(tops + (t0 + P >= S ? t0 + P - S : t0 + P) * csz, rank - 1);
+        return rank == 0 ? cl_addr(bots + b0 * csz, 0) : cl_addr(tops + (t0 + P >= S ? t0 + P - S : t0 + P) * csz, rank - 1);
     };
     auto leave_bot = [&](int t0, int b0) {
-        return rank == C - 1 ? jc_addr(tops + (t0 + P >= S ? t0 + P - S : t0 + P) * csz, rank)
-                             : jc_addr(bots + step(b0, -1) * csz, rank + 1);
+        return rank == C - 1 ? cl_addr(tops + (t0 + P >= S ? t0 + P - S : t0 + P) * csz, rank)
+                             : cl_addr(bots + step(b0, -1) * csz, rank + 1);
     };
     const bool moves = M > 1;
     // Q <- Q G with the rotations of table half h, the heads at t0 and b0
@@ -228,9 +204,9 @@ jacobi_cluster_kernel(int s, int P, int C, const T* __restrict__ Ain, T* __restr
                 if (jc_nonzero(sj) || lt || lb) {
                     const T qp = *cp, qq = *cq;
                     const T n_p = jc_lo(cj, sj, qp, qq), n_q = jc_hi(cj, sj, qp, qq);
-                    if (lt) jc_store(otop + row * sizeof(T), n_p);
+                    if (lt) cl_store(otop + row * sizeof(T), n_p);
                     else *cp = n_p;
-                    if (lb) jc_store(obot + row * sizeof(T), n_q);
+                    if (lb) cl_store(obot + row * sizeof(T), n_q);
                     else *cq = n_q;
                 }
             }
@@ -281,15 +257,15 @@ jacobi_cluster_kernel(int s, int P, int C, const T* __restrict__ Ain, T* __restr
                     }
                 }
                 if constexpr (CL) {
-                    jc_store(jc_addr(rc + i0 + j, k), c);
-                    jc_store(jc_addr(rs + i0 + j, k), sn);
+                    cl_store(cl_addr(rc + i0 + j, k), c);
+                    cl_store(cl_addr(rs + i0 + j, k), sn);
                 } else {
                     rc[j] = c;
                     rs[j] = sn;
                 }
             }
             if (r > 0) update_q((r - 1) & 1, step(th, -1), step(bh, 1));
-            jc_sync<CL>();
+            cl_sync<CL>();
             if (a_j < P) {
                 const int p = top_index(r, a_i), q = bot_index(r, a_i);
                 const double ci = rc[a_i];
@@ -319,15 +295,15 @@ jacobi_cluster_kernel(int s, int P, int C, const T* __restrict__ Ain, T* __restr
                             a_qq = s_from<T>(s_real(a_qq), 0.0);
                         }
                         if (lt) {
-                            jc_store(otop + p * sizeof(T), a_pp);
-                            jc_store(otop + q * sizeof(T), a_qp);
+                            cl_store(otop + p * sizeof(T), a_pp);
+                            cl_store(otop + q * sizeof(T), a_qp);
                         } else {
                             cp[p] = a_pp;
                             cp[q] = a_qp;
                         }
                         if (lb) {
-                            jc_store(obot + p * sizeof(T), a_pq);
-                            jc_store(obot + q * sizeof(T), a_qq);
+                            cl_store(obot + p * sizeof(T), a_pq);
+                            cl_store(obot + q * sizeof(T), a_qq);
                         } else {
                             cq[p] = a_pq;
                             cq[q] = a_qq;
@@ -335,7 +311,7 @@ jacobi_cluster_kernel(int s, int P, int C, const T* __restrict__ Ain, T* __restr
                     }
                 }
             }
-            jc_sync<CL>();
+            cl_sync<CL>();
             if (moves) {
                 th = step(th, 1);
                 bh = step(bh, -1);
@@ -367,7 +343,7 @@ jacobi_cluster_kernel(int s, int P, int C, const T* __restrict__ Ain, T* __restr
         for (int row = lane; row < s; row += 32) Qout[row + (int64_t)rk * s] = col[row];
     }
     if (rank == 0 && tid == 0 && info) info[0] = sweep;
-    jc_sync<CL>();  // no CTA leaves while another may still write to it
+    cl_sync<CL>();  // no CTA leaves while another may still write to it
 }
 
 template <class T>
