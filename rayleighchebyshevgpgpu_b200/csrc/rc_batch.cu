@@ -144,6 +144,8 @@ __global__ void __launch_bounds__(256, kBatchTileBlocksPerSm)
 batch_transpose_kernel(const BatchTable* __restrict__ T) {
     __shared__ double tile64[32][33];
     float(&tile32)[32][33] = *reinterpret_cast<float(*)[32][33]>(&tile64[0][0]);
+    float(&corr)[kCorrTileRows][33] = *reinterpret_cast<float(*)[kCorrTileRows][33]>(&tile64[0][0]);
+    static_assert(sizeof(corr) <= sizeof(tile64), "the correction tile shares the FP64 one");
     __shared__ int64_t ends[kMaxBatchJobs];
     const int nj = T->njobs;
     const int tid = threadIdx.x + threadIdx.y * blockDim.x;
@@ -161,7 +163,7 @@ batch_transpose_kernel(const BatchTable* __restrict__ T) {
             if (TO_RM) continue;
             const void* em = J.degree == 1 ? J.R : (J.degree % 2 == 0 ? J.bufA : J.bufB);
             corr_to_cm_tile<rc_corr_t>(J.n, J.s, (const rc_corr_t*)em, J.ld, J.V, J.ldv, J.coef,
-                                       J.a / (double)(J.degree + 1), r0, c0, tile32);
+                                       J.a / (double)(J.degree + 1), r0 / 32 * kCorrTileRows, c0, corr);
         } else if (TO_RM) {
             if (J.prec == P32) to_rm_tile<double, float>(J.n, J.s, J.V, J.ldv, (float*)J.bufA, J.ld, r0, c0, tile32);
             else to_rm_tile<double, double>(J.n, J.s, J.V, J.ldv, (double*)J.bufA, J.ld, r0, c0, tile64);
@@ -263,7 +265,7 @@ bool batch_job_describe_corr(const rc_ctx* ctx, const rc_op* op, double* V, int6
     J->s = s;
     J->degree = degree;
     J->vcta1 = (op->n + rows_per_cta - 1) / rows_per_cta;
-    J->tiles_x = (op->n + 31) / 32;
+    J->tiles_x = (op->n + kCorrTileRows - 1) / kCorrTileRows;
     J->tile1 = J->tiles_x * ((s + 31) / 32);
     J->rowptr = op->rowptr;
     J->colind = op->colind;

@@ -22,7 +22,7 @@ struct BatchJob {
     int64_t n, ld, ldv, s, degree;
     int64_t vcta0, vcta1;  // virtual CTAs of the degree steps
     int64_t tile0, tile1;  // virtual 32x32 tiles of the layout changes
-    int64_t tiles_x;       // row tiles, ceil(n / 32)
+    int64_t tiles_x;       // row tiles: of 32 rows, kCorrTileRows for the correction filter
     const int32_t* rowptr;
     const int32_t* colind;
     const void* vals;      // CSR values in the storage precision

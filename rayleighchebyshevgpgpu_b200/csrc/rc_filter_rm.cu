@@ -450,9 +450,9 @@ template <class TM, class TV>
 __global__ void __launch_bounds__(256)
 corr_to_cm_kernel(int64_t n, int64_t s, const TM* __restrict__ E, int64_t ld, TV* __restrict__ Vc, int64_t ldv,
                   const double* __restrict__ coef, double beta, const int* fail) {
-    __shared__ CorrTile<TM> tile[32][33];
+    __shared__ CorrTile<TM> tile[kCorrTileRows][33];
     const double nan = __longlong_as_double(0x7ff8000000000000ll);
-    corr_to_cm_tile<TM, TV>(n, s, E, ld, Vc, ldv, coef, fail && *fail ? nan : beta, (int64_t)blockIdx.x * 32,
+    corr_to_cm_tile<TM, TV>(n, s, E, ld, Vc, ldv, coef, fail && *fail ? nan : beta, (int64_t)blockIdx.x * kCorrTileRows,
                             (int64_t)blockIdx.y * 32, tile);
 }
 
@@ -623,7 +623,7 @@ static rc_status run_rm_corr(rc_ctx* ctx, const Pol& pol, int64_t n, TV* V, int6
                                                                  a / (double)(degree + 1), fail);
         }
     } else {
-        const dim3 tgrid((unsigned)((n + 31) / 32), (unsigned)((s + 31) / 32)), tblk(32, 8);
+        const dim3 tgrid((unsigned)((n + kCorrTileRows - 1) / kCorrTileRows), (unsigned)((s + 31) / 32)), tblk(32, 8);
         corr_to_cm_kernel<TM, TV><<<tgrid, tblk, 0, ctx->stream>>>(n, s, em, ld, V, ldv, coef,
                                                                    a / (double)(degree + 1), fail);
     }

@@ -103,3 +103,32 @@ def test_matrices_that_are_no_grid(change):
     for _ in range(3):
         x0, x1 = x1, -0.19 * (A @ x1) + 1.9 * x1 - x0
     np.testing.assert_allclose(b, (x1 / 5.0).T, rtol=0, atol=1e-13)
+
+
+@pytest.mark.parametrize("complex_", [False, True])
+@pytest.mark.parametrize("dims", [(63, 2, 1), (64, 3, 1), (13, 5, 3), (8, 8, 9)])
+@pytest.mark.parametrize("s", [1, 9, 32, 33, 70])
+def test_correction_exit_is_the_same_for_every_alignment(ctx, complex_, dims, s):
+    """The last step reads and writes pairs of rows where they are 16-byte aligned: even and odd leading dimensions and a
+    block that starts one entry off give the same bits, and nothing outside the block changes."""
+    import torch
+    kind = 5 if dims[2] == 1 else 7
+    n = int(np.prod(dims))
+    op = _operator(ctx, "stencil", kind, complex_, dims)
+    rng = np.random.default_rng(s)
+    V = rng.standard_normal((s, n)) + (1j * rng.standard_normal((s, n)) if complex_ else 0)
+    lam = rng.uniform(5.0, 7.0, s)
+    out = []
+    for pad, shift in ((0, 0), (1, 0), (2, 1)):
+        ld = n + pad
+        buf = torch.full((s * ld + 8,), 7.5, dtype=torch.complex128 if complex_ else torch.float64, device="cuda")
+        Vd = buf[shift:shift + s * ld].view(s, ld)
+        Vd[:, :n] = torch.from_numpy(V)
+        torch.cuda.synchronize()
+        R.filter_correction(ctx, op, Vd, s, lam, 4, -0.1, 1.9, ld=ld)
+        ctx.synchronize()
+        out.append(Vd[:, :n].cpu().numpy())
+        Vd[:, :n] = 7.5
+        assert (buf == 7.5).all()
+    assert np.array_equal(out[0], out[1]) and np.array_equal(out[0], out[2])
+    op.close()
