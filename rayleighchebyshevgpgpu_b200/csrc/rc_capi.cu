@@ -14,6 +14,7 @@
 #include "rc_common.cuh"
 #include "rc_cpoly.h"
 #include "rc_internal.h"
+#include "rc_batch.h"
 #include "rc_tile.h"
 
 namespace rcb {
@@ -174,6 +175,7 @@ rc_status rc_ctx_destroy(rc_ctx* ctx) {
     cudaStreamSynchronize(ctx->stream);
     if (ctx->host_small) cudaFreeHost(ctx->host_small);
     if (ctx->host_eigh) cudaFreeHost(ctx->host_eigh);
+    rcb::batch_runner_destroy(ctx->batch_runner);
     for (cudaEvent_t e : ctx->step_events) cudaEventDestroy(e);
     if (ctx->own_stream) cudaStreamDestroy(ctx->own_stream);
     delete ctx;

@@ -36,6 +36,10 @@ struct DevBuf {
     size_t bytes = 0;
 };
 
+namespace rcb {
+struct BatchRunner;
+}
+
 struct rc_ctx {
     int device = 0;
     cudaStream_t stream = nullptr;
@@ -49,6 +53,7 @@ struct rc_ctx {
     double* host_small = nullptr;
     size_t host_small_bytes = 0;
     // and for rc_small_eigh's matrices (its own: an operator callback may call it during a solve)
+    rcb::BatchRunner* batch_runner = nullptr;  // of rc_filter_correction_batch (rc_corrapi.cu), from its first call on
     void* host_eigh = nullptr;
     size_t host_eigh_bytes = 0;
     int sm_count = 148;
