@@ -225,7 +225,7 @@ rc_status rc_cholqr(rc_ctx* ctx, int dtype, void* V, int64_t ld, int64_t n, int6
 rc_status rc_rayleigh_ritz(rc_ctx* ctx, const rc_op* op, void* V, void* W, int64_t ld, int64_t s,
                            int64_t res_count, double* evals, double* residuals, void* Q);
 
-/* Eigen-decomposition of a small Hermitian matrix on the GPU (one-CTA parallel Jacobi),
+/* Eigen-decomposition of a small Hermitian matrix on the GPU (parallel Jacobi),
  * ascending eigenvalues, eigenvectors in the columns of Q. H, Q, evals: HOST arrays.
  * Replaces DSYEV/ZHPEVX (RayleighChebyshevLMCuda.h:614,618) and JacobiDiagonalizer. */
 rc_status rc_small_eigh(rc_ctx* ctx, int dtype, int64_t s, const void* H, double* evals, void* Q);

@@ -30,9 +30,11 @@ constexpr int CM_THREADS = 512;
 constexpr int CM_COPIES = 8;                      // copies per thread and column, at most
 constexpr int CM_MAX_BOX = CM_COPIES * CM_THREADS;
 constexpr size_t CM_MAX_SMEM = 224 * 1024;
-// Smallest block for the tiles: 24^3 and 24 columns (2.7 MB) took 15.5 us against the gather's 13.1, 24^3 and 48 columns
-// (5.3 MB) 17.5 against 21.4, 32^3 and 32 columns (8.4 MB) 15.0 against 16.9. Fewer than 8 columns leave no ring to fill.
-constexpr int64_t kCmMinBytes = 5ll << 20;
+// Smallest block for the tiles. Smaller ones stay in L2, where the gather kernels read at ease and a tile's start shows:
+// complex CSR 40^3 x 24 (23 MB) 18.9 -> 25.5 us, 5 points 333 x 400 x 24 (26 MB) 16.8 -> 23.1, stencil 40^3 x 53 (27 MB)
+// 18.9 -> 21.1, complex 56 x 61 x 50 x 13 (36 MB) 23.0 -> 24.1; no measured block beyond was slower (48^3 x 53, 45 MB; 40^3 x 96, 49 MB; 100^3 x 16, 128 MB 149 -> 79).
+// Fewer than 8 columns leave no ring to fill.
+constexpr int64_t kCmMinBytes = 40ll << 20;
 
 enum { CK_STENCIL7 = 0, CK_CSR7 = 1, CK_STENCIL5 = 2 };  // 5 points: the grid's y is the kernel's z
 template <class T>

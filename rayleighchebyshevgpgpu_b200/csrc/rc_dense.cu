@@ -1,6 +1,6 @@
 // rc_dense.cu -- FP64 (c128) dense kernels of the orthonormalisation and Rayleigh-Ritz steps.
 //
-//  gram      C = X^H Y for tall-skinny n x m and n x nc blocks: split over row chunks, each
+//  gram      C = X^H Y for tall-skinny n x m and n x nc blocks that rc_gram.cu does not take: split over row chunks, each
 //            CTA accumulates a 64x64 output tile in registers from shared-memory K-tiles,
 //            partial tiles are summed by a second kernel in a fixed order (deterministic).
 //            Replaces cublas{D,Z}gemm(OP_T/OP_C, OP_N) (RayleighChebyshevLMCuda.h:2139-2161).
@@ -8,9 +8,9 @@
 //            (W*Q next to V*Q) with the residual ||W_c - lam_c V_c||^2 reduced in the epilogue.
 //            Replaces cublas{D,Z}gemm(OP_N,OP_N) + normalize + memcpy + the second SpMM +
 //            the residuals kernel (RayleighChebyshevLMCuda.h:2178-2285, cuda_kernels.cu:307-382).
-//  chol      Cholesky of a column-scaled Gram matrix and the inverse of its factor (one CTA);
+//  chol      Cholesky of a column-scaled Gram matrix and the inverse of its factor (more than 192 columns);
 //            with xt it forms CholeskyQR, replacing cusolverDn geqrf+orgqr (:1979-2107).
-//  eigh      one-CTA parallel cyclic Jacobi for a small Hermitian matrix, replacing host
+//  eigh      parallel cyclic Jacobi for a small Hermitian matrix that rc_jacobi.cu does not take, replacing host
 //            DSYEV/ZHPEVX (:570-642) and JacobiDiagonalizer.
 #include <algorithm>
 #include <cmath>

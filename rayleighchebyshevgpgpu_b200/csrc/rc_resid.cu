@@ -400,7 +400,7 @@ rc_status resid_block(rc_ctx* ctx, const rc_op* op, const void* Yrm, int64_t ld,
     double* part = nullptr;
     int64_t parts = 0;
     rc_status st = RC_OK;
-    if (tile_supported(ctx, op, op->dtype == RC_COMPLEX128 ? TT_C128 : TT_F64, ld) &&
+    if (tile_supported(ctx, op, op->dtype == RC_COMPLEX128 ? TT_C128 : TT_F64, ld, true) &&
         tile_resid(ctx, op, Yrm, ld, s, lam, res_count, R, ldr, &part, &parts, &st)) {
         RC_TRY(st);
         RC_CU(ctx, cudaGetLastError());

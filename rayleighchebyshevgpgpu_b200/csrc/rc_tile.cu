@@ -36,10 +36,23 @@ namespace rcb {
 
 namespace {
 
-// Smallest block (bytes) for which the tile kernels are taken for 7 points: below, both forms take a launch's latency
-// (24^3, 24 FP64 columns, 2.7 MB: 68 us for 5 steps either way; 24^3, 96 columns: 88 -> 73 us). 27 points: always
-// (8^3, 24 columns: 303 -> 69 us).
-constexpr int64_t kTileMinBytes = 4ll << 20;
+// Smallest block (bytes) for which the tile kernels are taken for 7 points. Below, a step is a launch's latency either
+// way, or the panels and units of a small grid leave SMs without work; the lines are where no measured grid (12 x 23 x 54
+// to 61 x 53 x 67; 8, 24, 53 and 96 columns) was slower beyond them. Filters of 10 steps, gather -> tiles, us:
+//   FP64      CSR 40^3 x 24 (12 MB) 177 -> 117; stencil 40^3 x 53 (26 MB) 207 -> 281, 48^3 x 53 (45 MB) 394 -> 319
+//   c128      CSR 20^3 x 53 (6 MB) 121 -> 155, 12 x 48 x 64 x 53 (30 MB) 351 -> 373, 48^3 x 24 (40 MB) 474 -> 291;
+//             stencil 16 x 40 x 40 x 8 (3 MB) 93 -> 102, 32^3 x 53 (26 MB) 256 -> 203
+//   bfloat16  CSR 32^3 x 24 (1.5 MB) 131 -> 182, 48^3 x 53 (11 MB) 246 -> 189; stencil 48^3 x 24 (5 MB) 177 -> 156
+//   pairs     CSR 40^3 x 96 (23 MB) 412 -> 452; stencil 94 MB of c128 376 -> 396
+// 27 points: always (8^3, 24 columns: 303 -> 69).
+constexpr int64_t tile_min_bytes(TileType t, bool csr, bool resid) {
+    switch (t) {
+        case TT_F64: return csr || resid ? 4ll << 20 : 32ll << 20;
+        case TT_C128: return csr ? 32ll << 20 : 16ll << 20;
+        case TT_BF16: return csr ? 6ll << 20 : 4ll << 20;
+        default: return 32ll << 20;
+    }
+}
 
 enum { TK_STENCIL7 = 0, TK_CSR7 = 1, TK_STENCIL27 = 2 };
 // Points along y per thread. 27 points: the sums of three planes of four points spill at 128 registers.
@@ -653,12 +666,13 @@ bool tile_launch(rc_ctx* ctx, const TileArgs& A, const TileMaps& M, const TileSt
 
 }  // namespace
 
-bool tile_supported(const rc_ctx* ctx, const rc_op* op, TileType type, int64_t ld) {
+bool tile_supported(const rc_ctx* ctx, const rc_op* op, TileType type, int64_t ld, bool resid) {
     if (!ctx->tile) return false;
     const Structure S = structure(op, type == TT_BF16 || type == TT_BF16C);
     if (S.kind < 0 || (op->dtype == RC_COMPLEX128) != (type == TT_C128 || type == TT_BF16C)) return false;
     if (S.kind == TK_STENCIL27 && op->dtype == RC_COMPLEX128) return false;
-    return ctx->tile > 1 || S.kind == TK_STENCIL27 || op->n * ld * tile_elem(type) >= kTileMinBytes;
+    return ctx->tile > 1 || S.kind == TK_STENCIL27 ||
+           op->n * ld * tile_elem(type) >= tile_min_bytes(type, S.kind == TK_CSR7, resid);
 }
 
 template <class TS, class TC, class TM, bool SRC>

@@ -8,7 +8,7 @@ namespace rcb {
 enum TileType { TT_F64 = 0, TT_C128, TT_BF16, TT_BF16C };
 
 // Whether the operator has the structure and the block (row length ld) the size for the tile kernels.
-bool tile_supported(const rc_ctx* ctx, const rc_op* op, TileType type, int64_t ld);
+bool tile_supported(const rc_ctx* ctx, const rc_op* op, TileType type, int64_t ld, bool resid = false);
 // y = alpha A x + beta x + gamma z (+ sig[c] src): rm_step_rows' step; z may be null, src goes with TT_BF16*.
 // False (nothing launched) when a pointer is not 16-byte aligned or the driver refuses a tensor map.
 bool tile_step(rc_ctx* ctx, const rc_op* op, TileType type, int64_t ld, const void* x, const void* z, void* y, double alpha,
