@@ -576,9 +576,23 @@ Structure structure(const rc_op* op, bool fp32) {
 }
 constexpr int tile_elem(TileType t) { return t == TT_BF16 ? 2 : (t == TT_BF16C ? 4 : (t == TT_F64 ? 8 : 16)); }
 
+// Whether the plan is better than the gather kernels' form for 7 points: the waste of the grid's edges and halos (traffic
+// against that of the points alone) and the threads of a CTA, of which there is one per SM. Filters of 10 steps on
+// narrow and ragged grids, 3 to 40 columns, gather -> tiles, us: FP64 CSR 18 x 11 x 4000 x 12 (waste 2.0, 96 threads)
+// 924 -> 1092, 37 x 70 x 200 x 40 (1.36, 160) 1596 -> 1229, the stencil 1117 -> 1269, 61 x 53 x 250 x 24 (1.25, 384)
+// 1076 -> 854; bfloat16 CSR 24 x 24 x 1000 x 24 (1.39, 288) 504 -> 453, the stencil 417 -> 444; 37 x 70 x 200 x 24 (1.36,
+// 96) 466 -> 511; pairs 18 x 11 x 4000 x 12 (2.03, 288) 701 -> 952. One slice a row of bfloat16 is too little for a TMA
+// box's lines (100 x 90 x 60 x 8: 213 -> 290).
+bool tile_pays(TileType type, bool csr, double waste, int threads, int nseg) {
+    const bool bf16 = type == TT_BF16 || type == TT_BF16C;
+    if (bf16 && nseg < 2) return false;
+    if (waste > (csr && type != TT_BF16C ? 1.45 : 1.3)) return false;
+    return threads >= (csr && !bf16 ? 160 : (type == TT_C128 ? 256 : 192));
+}
+
 // Tiles, slots and units for blocks of `slices` 16-byte slices a row; zops planes beside x, wbytes of weights a row.
-bool tile_plan(const rc_ctx* ctx, const Structure& S, int slices, int zops, int wbytes, TileArgs* out, unsigned* grid,
-               size_t* smem) {
+bool tile_plan(const rc_ctx* ctx, const Structure& S, TileType type, int slices, int zops, int wbytes, TileArgs* out,
+               unsigned* grid, size_t* smem) {
     TileArgs A = {};
     A.nx = (int)S.nx;
     A.ny = (int)S.ny;
@@ -609,6 +623,9 @@ bool tile_plan(const rc_ctx* ctx, const Structure& S, int slices, int zops, int 
             }
         }
     if (!A.tx) return false;
+    if (ctx->tile == 1 && S.kind != TK_STENCIL27 &&
+        !tile_pays(type, S.kind == TK_CSR7, least / ((double)A.nx * A.ny * (2.0 + zops)), A.tx * A.ty / R * A.nseg, A.nseg))
+        return false;
     A.xbytes = up(A.nseg * 16 * (A.tx + 2) * (A.ty + 2));
     A.zbytes = up(A.nseg * 16 * A.tx * A.ty);
     A.cbytes = up(wbytes * A.tx * A.ty);
@@ -686,7 +703,7 @@ static bool tile_step_t(rc_ctx* ctx, const rc_op* op, TileType type, int64_t ld,
     const int zops = (z ? 1 : 0) + (SRC ? 1 : 0);
     const int wb = st.kind == TK_CSR7 ? (int)sizeof(RowWeights<TC>) : 0;
     const int64_t words = ld * (int64_t)sizeof(TM) / 4;
-    if (!tile_plan(ctx, st, (int)(words / 4), zops, wb, &A, &grid, &smem)) return false;
+    if (!tile_plan(ctx, st, type, (int)(words / 4), zops, wb, &A, &grid, &smem)) return false;
     A.ld = ld;
     A.has_z = z != nullptr;
     A.off = op->offdiag;
@@ -737,7 +754,7 @@ static bool tile_resid_t(rc_ctx* ctx, const rc_op* op, const void* Y, int64_t ld
     size_t smem;
     const int wb = st.kind == TK_CSR7 ? (int)sizeof(RowWeights<T>) : 0;
     const int64_t words = ld * (int64_t)sizeof(T) / 4;
-    if (!tile_plan(ctx, st, (int)(words / 4), 0, wb, &A, &grid, &smem)) return false;
+    if (!tile_plan(ctx, st, IsComplex<T>::value ? TT_C128 : TT_F64, (int)(words / 4), 0, wb, &A, &grid, &smem)) return false;
     A.ld = ld;
     A.off = op->offdiag;
     A.diag = op->diag64;
