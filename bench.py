@@ -68,7 +68,8 @@ def profile_dram_bytes_per_row():
     """DRAM bytes per grid row of one filter degree-step, from the committed ncu summaries
     (lines "dram-bytes-per-row fp32=<B> fp64=<B>" and "dram-bytes-per-row corr=<B>"), or None."""
     out = {}
-    for name in ("rm_step_kernel_csr_96cube_s96.md", "rm_step_src_kernel_csr_96cube_s96.md"):
+    for name in ("rm_step_kernel_csr_96cube_s96.md", "rm_step_src_kernel_csr_96cube_s96.md",
+                 "tile_kernel_csr_96cube_s96.md"):
         try:
             for line in open(os.path.join(ROOT, "profiles", name)):
                 if line.startswith("dram-bytes-per-row"):
@@ -433,17 +434,17 @@ def run_ours(args):
     e2e_value = replicas.job_rate(P.k, world, max_over_ranks(statistics.median(e2e_t)))
     assert np.array_equal(res_e.evals, res_mixed.evals)
 
-    # ---- roofline of the dominant kernel: the fused filter degree-step (rm_step_kernel) ----
-    # Algorithmic bytes of one degree-step over the n x s block: the matrix once (values + column
-    # indices + row pointers) and three block passes (read x_{k-1}, read x_{k-2}, write x_k); the
-    # correction filter's step (rm_step_src_kernel) also reads the residual block: four passes of
+    # ---- roofline of the dominant kernel: the fused filter degree-step (tile_kernel) ----
+    # Algorithmic bytes of one degree-step over the n x s block: the matrix once and three block passes (read x_{k-1}, read x_{k-2}, write x_k); the
+    # correction filter's step also reads the residual block: four passes of
     # its storage type (bfloat16 or FP32, info.correction_element_bytes).
     # The step time is the CUDA-event time of the degree-step launches inside the timed solves
     # (info.time_filter_steps_ms, transposes excluded). Degree-1 filters (column-major path, at
     # most a few per solve) are counted in degree_steps but not timed, a < 0.1 % overstatement.
     nnz = ci.size
-    b_a32 = nnz * (4 + 4) + (P.n + 1) * 4
-    b_a64 = nnz * (8 + 4) + (P.n + 1) * 4
+    # (the steps read the rows' packed weights, eight to a row, in place of the CSR arrays)
+    b_a32 = P.n * 8 * 4
+    b_a64 = P.n * 8 * 8
     bytes_fp32_step = b_a32 + 3 * P.n * s * 4
     ceb = int(infos[-1].get("correction_element_bytes", 4) or 4)
     bytes_corr_step = b_a32 + 4 * P.n * s * ceb
@@ -518,7 +519,7 @@ def run_ours(args):
                                                            "time_ortho_ms", "time_eigenvalue_ms")} if info64 else None},
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                      "frac": (achieved / peak) if achieved else None, "traffic": traffic,
-                     "peak_source": peak_src, "kernel": "rm_step_kernel + rm_step_src_kernel (fused filter degree-steps, CSR)",
+                     "peak_source": peak_src, "kernel": "tile_kernel (fused filter degree-steps, CSR rows of a 7-point grid)",
                      "algorithmic_bytes_per_launch": alg_bytes / fsteps if fsteps else None,
                      "launches": fsteps, "fp64_launches": f64steps, "correction_launches": csteps,
                      "bytes_per_launch_fp32": bytes_fp32_step, "bytes_per_launch_correction": bytes_corr_step,
