@@ -435,9 +435,10 @@ def run_ours(args):
     assert np.array_equal(res_e.evals, res_mixed.evals)
 
     # ---- roofline of the dominant kernel: the fused filter degree-step (tile_kernel) ----
-    # Algorithmic bytes of one degree-step over the n x s block: the matrix once and three block passes (read x_{k-1}, read x_{k-2}, write x_k); the
-    # correction filter's step also reads the residual block: four passes of
-    # its storage type (bfloat16 or FP32, info.correction_element_bytes).
+    # Algorithmic bytes of one degree-step over the n x s block: the matrix once and three block
+    # passes (read x_{k-1}, read x_{k-2}, write x_k); the correction filter's step also reads the
+    # residual block: four passes of its storage type (bfloat16 or FP32,
+    # info.correction_element_bytes).
     # The step time is the CUDA-event time of the degree-step launches inside the timed solves
     # (info.time_filter_steps_ms, transposes excluded). Degree-1 filters (column-major path, at
     # most a few per solve) are counted in degree_steps but not timed, a < 0.1 % overstatement.
