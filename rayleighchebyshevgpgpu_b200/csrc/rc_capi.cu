@@ -639,7 +639,8 @@ rc_status rc_small_eigh(rc_ctx* ctx, int dtype, int64_t s, const void* H, double
     // one pinned copy each way (H; evals, sweeps and Q together): staged by the driver from pageable memory, the
     // four copies took 55 of the 200 us of a 24 x 24 call
     const size_t mat = (size_t)s * s * elem_bytes(dtype, P64);
-    const size_t head = ((size_t)s * 8 + 8 + 255) / 256 * 256;
+    // eigenvalues, then four words: the sweep count, and three that the grid kernel's barrier polls to its end
+    const size_t head = ((size_t)s * 8 + 4 * sizeof(int) + 255) / 256 * 256;
     void* sm = nullptr;
     RC_TRY(rc_slot(ctx, S_SMALL, 2 * mat + head + 256, &sm));
     const size_t need = head + mat;
