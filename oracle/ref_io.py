@@ -23,14 +23,15 @@ def ref_available() -> bool:
 
 
 def reference_present(reference_dir: str | None = None) -> bool:
-    return os.path.isdir(reference_dir or REFERENCE_DIR)
+    # a mount point without the sources behind it counts as absent
+    return os.path.isfile(os.path.join(reference_dir or REFERENCE_DIR, "RayleighChebyshevLM.h"))
 
 
 def build_ref(reference_dir: str | None = None, targets=("_ref/ref_harness",)) -> bool:
     """Compile the reference harness (and any other oracle/Makefile targets) from the reference
     sources, when they are present."""
     reference_dir = reference_dir or REFERENCE_DIR
-    if not os.path.isdir(reference_dir):
+    if not reference_present(reference_dir):
         return ref_available()
     r = subprocess.run(["make", "-C", ORACLE_DIR, f"REF={reference_dir}", *targets], capture_output=True, text=True)
     if r.returncode != 0:
