@@ -236,6 +236,13 @@ static rc_status dev_copy(rc_ctx* ctx, void** dst, const void* src, size_t bytes
     ctx->op_bytes += (int64_t)bytes;
     return RC_OK;
 }
+// The copies go through the default stream, and from pageable memory they may return once the data is staged. No other
+// stream here waits for the default one (contexts' own streams are non-blocking), so an operator is handed out, and its
+// arrays are read, only when they have landed.
+static rc_status dev_copies_landed(rc_ctx* ctx) {
+    RC_CU(ctx, cudaStreamSynchronize(cudaStreamLegacy));
+    return RC_OK;
+}
 
 // Whether the rows are those of a 7-point stencil on a grid of at least two points each way: row 0 holds the columns
 // 0, 1, L and P with L | P | n, and row i the diagonal and exactly the neighbours that lie in the grid, columns
@@ -333,13 +340,14 @@ rc_status rc_op_csr_create(rc_ctx* ctx, int dtype, int64_t n, int64_t nnz, const
     rc_status st = dev_copy(ctx, (void**)&op->rowptr, rowptr, (size_t)(n + 1) * 4, op);
     if (st == RC_OK) st = dev_copy(ctx, (void**)&op->colind, colind, (size_t)nnz * 4, op);
     if (st == RC_OK) st = dev_copy(ctx, &op->vals64, vals, (size_t)nnz * vsz, op);
+    if (st == RC_OK) st = dev_copies_landed(ctx);
     if (st == RC_OK && op->gx > 0) {
         size_t b = 0;
         st = rcb::tile_pack(ctx, op, false, op->vals64, &op->pack64, &b);
         if (st == RC_OK) {
             op->bytes += (int64_t)b;
             ctx->op_bytes += (int64_t)b;
-            // other contexts' streams may use the operator as soon as it exists (its other arrays are copied in order)
+            // other contexts' streams may use the operator as soon as it exists
             if (cudaStreamSynchronize(ctx->stream) != cudaSuccess)
                 st = rc_fail(ctx, RC_ERR_CUDA, "rc_op_csr_create: packing the weights failed");
         }
@@ -392,6 +400,7 @@ rc_status rc_op_stencil_create(rc_ctx* ctx, int dtype, int kind, int64_t nx, int
         st = dev_copy(ctx, &op->phase64, p64.data(), p64.size() * sizeof(double), op);
         if (st == RC_OK) st = dev_copy(ctx, &op->phase32, p32.data(), p32.size() * sizeof(float), op);
     }
+    if (st == RC_OK) st = dev_copies_landed(ctx);
     if (st != RC_OK) {
         rc_op_destroy(op);
         return st;
