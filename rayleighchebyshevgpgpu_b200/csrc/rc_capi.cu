@@ -27,6 +27,19 @@ rc_status rc_fail(rc_ctx* ctx, rc_status st, const std::string& msg) {
     return st;
 }
 
+cudaError_t rc_device_alloc(rc_ctx* ctx, void** out, size_t bytes) {
+    cudaError_t e = cudaMalloc(out, bytes);
+    if (e == cudaErrorMemoryAllocation && rcb::tile_weights_release(ctx)) {
+        cudaGetLastError();
+        e = cudaMalloc(out, bytes);
+    }
+    if (e != cudaSuccess) {
+        cudaGetLastError();
+        *out = nullptr;
+    }
+    return e;
+}
+
 rc_status rc_slot(rc_ctx* ctx, int slot, size_t bytes, void** out) {
     if ((int)ctx->slots.size() < S_COUNT) ctx->slots.resize(S_COUNT);
     DevBuf& b = ctx->slots[slot];
@@ -44,7 +57,7 @@ rc_status rc_slot(rc_ctx* ctx, int slot, size_t bytes, void** out) {
         // round up to 2 MiB so repeated small growth does not thrash the allocator
         const size_t want = ((bytes + (2u << 20) - 1) / (2u << 20)) * (2u << 20);
         const cudaError_t e = ctx->pool ? cudaMallocFromPoolAsync(&b.ptr, want, ctx->pool, ctx->stream)
-                                        : cudaMalloc(&b.ptr, want);
+                                        : rc_device_alloc(ctx, &b.ptr, want);
         if (e != cudaSuccess) {
             cudaGetLastError();
             b.ptr = nullptr;
@@ -100,8 +113,8 @@ static void op_release(rc_op* op) {
     if (op->colind) cudaFree(op->colind);
     if (op->vals64) cudaFree(op->vals64);
     if (op->vals32) cudaFree(op->vals32);
-    if (op->pack64) cudaFree(op->pack64);
-    if (op->pack32) cudaFree(op->pack32);
+    for (auto& w : op->pack)
+        if (w.load()) cudaFree(w.load());
     if (op->diag64) cudaFree(op->diag64);
     if (op->diag32) cudaFree(op->diag32);
     if (op->phase64) cudaFree(op->phase64);
@@ -227,8 +240,7 @@ rc_status rc_ctx_device_bytes(rc_ctx* ctx, int64_t* bytes) {
 // Operator arrays carry 64 bytes of tail padding: the staged step kernels copy 16-byte aligned
 // spans of them, which may reach up to 15 bytes past the last element.
 static rc_status dev_copy(rc_ctx* ctx, void** dst, const void* src, size_t bytes, rc_op* op) {
-    if (cudaMalloc(dst, bytes + 64) != cudaSuccess) {
-        cudaGetLastError();
+    if (rc_device_alloc(ctx, dst, bytes + 64) != cudaSuccess) {
         return rc_fail(ctx, RC_ERR_NOMEM, "cudaMalloc for operator storage failed");
     }
     if (bytes) RC_CU(ctx, cudaMemcpy(*dst, src, bytes, cudaMemcpyHostToDevice));
@@ -341,17 +353,6 @@ rc_status rc_op_csr_create(rc_ctx* ctx, int dtype, int64_t n, int64_t nnz, const
     if (st == RC_OK) st = dev_copy(ctx, (void**)&op->colind, colind, (size_t)nnz * 4, op);
     if (st == RC_OK) st = dev_copy(ctx, &op->vals64, vals, (size_t)nnz * vsz, op);
     if (st == RC_OK) st = dev_copies_landed(ctx);
-    if (st == RC_OK && op->gx > 0) {
-        size_t b = 0;
-        st = rcb::tile_pack(ctx, op, false, op->vals64, &op->pack64, &b);
-        if (st == RC_OK) {
-            op->bytes += (int64_t)b;
-            ctx->op_bytes += (int64_t)b;
-            // other contexts' streams may use the operator as soon as it exists
-            if (cudaStreamSynchronize(ctx->stream) != cudaSuccess)
-                st = rc_fail(ctx, RC_ERR_CUDA, "rc_op_csr_create: packing the weights failed");
-        }
-    }
     if (st != RC_OK) {
         rc_op_destroy(op);
         return st;
@@ -433,7 +434,7 @@ rc_status rc_op_destroy(rc_op* op) {
     if (ctx) {
         cudaSetDevice(ctx->device);
         cudaStreamSynchronize(ctx->stream);
-        ctx->op_bytes -= op->bytes;
+        ctx->op_bytes -= op->bytes + op->pack_bytes;
         for (size_t i = 0; i < ctx->ops.size(); ++i)
             if (ctx->ops[i] == op) {
                 ctx->ops.erase(ctx->ops.begin() + i);

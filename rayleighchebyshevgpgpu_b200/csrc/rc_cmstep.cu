@@ -262,14 +262,14 @@ bool cm_plan(const rc_ctx* ctx, int kind, int64_t nx, int64_t ny, int64_t nz, in
 
 template <class T, int KIND>
 rc_status cm_launch(rc_ctx* ctx, const rc_op* op, const StepArgs& a, T alpha, T beta, T gamma, const double* lam,
-                    int64_t res_count, const CmArgs& A, dim3 grid, const CUtensorMap* map, double* part) {
+                    int64_t res_count, const CmArgs& A, dim3 grid, const CUtensorMap* map, double* part, const void* weights) {
     const size_t smem = (size_t)cm_slots<T>() * A.slot * sizeof(T);
     const CUtensorMap none = {};
     const double theta = 2.0 * 3.14159265358979323846 * op->flux;
     auto run = [&](auto kern) -> rc_status {
         RC_CU(ctx, allow_max_smem(ctx, kern));
         kern<<<grid, CM_THREADS, smem, ctx->stream>>>(A, map ? *map : none, (const T*)a.x, a.ldx, (const T*)a.z, a.ldz, (T*)a.y, a.ldy,
-                                                      alpha, beta, gamma, a.scale, (const RowWeights<T>*)op->pack64,
+                                                      alpha, beta, gamma, a.scale, (const RowWeights<T>*)weights,
                                                       op->diag64, op->offdiag, theta, lam, (int)res_count, part);
         ctx->launches++;
         RC_CU(ctx, cudaGetLastError());
@@ -282,7 +282,7 @@ rc_status cm_launch(rc_ctx* ctx, const rc_op* op, const StepArgs& a, T alpha, T 
 }
 
 template <class T>
-rc_status cm_step_t(rc_ctx* ctx, const rc_op* op, const StepArgs& a, const double* lam, int64_t res_count, double** part,
+rc_status cm_step_t(rc_ctx* ctx, rc_op* op, const StepArgs& a, const double* lam, int64_t res_count, double** part,
                     int64_t* parts, bool* done) {
     const int kind = op->kind == 0 ? CK_CSR7 : (op->skind == 7 ? CK_STENCIL7 : CK_STENCIL5);
     const int64_t nx = kind == CK_CSR7 ? op->gx : op->nx;
@@ -303,7 +303,6 @@ rc_status cm_step_t(rc_ctx* ctx, const rc_op* op, const StepArgs& a, const doubl
         if (!tma_map_words_4d(&map, a.x, dims, box, a.ldx * W)) return RC_OK;
     }
     const CUtensorMap* mp = tma ? &map : nullptr;
-    *done = true;
     double* pt = nullptr;
     if (res_count > 0) {
         void* p = nullptr;
@@ -311,6 +310,10 @@ rc_status cm_step_t(rc_ctx* ctx, const rc_op* op, const StepArgs& a, const doubl
         *part = pt = (double*)p;
         *parts = grid.x;
     }
+    // (after the allocation, which may take them back when memory is short)
+    const void* weights = kind == CK_CSR7 ? tile_weights(ctx, op, false, op->n * a.s * (int64_t)sizeof(T)) : nullptr;
+    if (kind == CK_CSR7 && !weights) return RC_OK;
+    *done = true;
     T alpha, beta, gamma;
     if constexpr (IsComplex<T>::value) {
         alpha = make_double2(a.alpha[0], a.alpha[1]);
@@ -321,21 +324,21 @@ rc_status cm_step_t(rc_ctx* ctx, const rc_op* op, const StepArgs& a, const doubl
         beta = a.beta[0];
         gamma = a.gamma[0];
         if (kind == CK_STENCIL5)
-            return cm_launch<T, CK_STENCIL5>(ctx, op, a, alpha, beta, gamma, lam, res_count, A, grid, mp, pt);
+            return cm_launch<T, CK_STENCIL5>(ctx, op, a, alpha, beta, gamma, lam, res_count, A, grid, mp, pt, weights);
     }
     if (kind == CK_CSR7)
-        return cm_launch<T, CK_CSR7>(ctx, op, a, alpha, beta, gamma, lam, res_count, A, grid, mp, pt);
-    return cm_launch<T, CK_STENCIL7>(ctx, op, a, alpha, beta, gamma, lam, res_count, A, grid, mp, pt);
+        return cm_launch<T, CK_CSR7>(ctx, op, a, alpha, beta, gamma, lam, res_count, A, grid, mp, pt, weights);
+    return cm_launch<T, CK_STENCIL7>(ctx, op, a, alpha, beta, gamma, lam, res_count, A, grid, mp, pt, weights);
 }
 
 }  // namespace
 
-rc_status cm_step(rc_ctx* ctx, const rc_op* op, const StepArgs& a, const double* lam, int64_t res_count, double** part,
+rc_status cm_step(rc_ctx* ctx, rc_op* op, const StepArgs& a, const double* lam, int64_t res_count, double** part,
                   int64_t* parts, bool* done) {
     *done = false;
     const bool cplx = op->dtype == RC_COMPLEX128;
     if (!ctx->tile || a.cp != P64 || a.xp != P64 || a.yp != P64 || (a.z && a.zp != P64)) return RC_OK;
-    if (op->kind == 0 ? !(op->gx > 0 && op->pack64 && ctx->csr_variant == 0)
+    if (op->kind == 0 ? !(tile_rows(ctx, op, false) && ctx->csr_variant == 0)
                       : !(op->kind == 1 && (op->skind == 7 || (op->skind == 5 && !cplx))))
         return RC_OK;
     if (op->n > 0x7fffffff || a.s > 0x7fffffff) return RC_OK;  // row numbers of 31 bits

@@ -347,29 +347,18 @@ rc_status ensure_fp32(rc_ctx* ctx, rc_op* op) {
     if (op->kind == 0 && op->vals32 == nullptr) {
         const int64_t cnt = op->nnz * (op->dtype == RC_COMPLEX128 ? 2 : 1);
         void* p = nullptr;
-        if (cudaMalloc(&p, (size_t)cnt * 4 + 64) != cudaSuccess)  // tail padding as the other operator arrays
+        if (rc_device_alloc(ctx, &p, (size_t)cnt * 4 + 64) != cudaSuccess)  // tail padding as the other operator arrays
             return rc_fail(ctx, RC_ERR_NOMEM, "cudaMalloc failed for FP32 operator values");
         cvt_f64_f32_kernel<<<4 * kB200Sms, 256, 0, ctx->stream>>>((const double*)op->vals64, (float*)p, cnt);
         ctx->launches++;
         RC_CU(ctx, cudaGetLastError());
-        if (op->gx > 0) {
-            size_t b = 0;
-            const rc_status st = tile_pack(ctx, op, true, p, &op->pack32, &b);
-            if (st != RC_OK) {
-                cudaStreamSynchronize(ctx->stream);
-                cudaFree(p);
-                return st;
-            }
-            op->bytes += (int64_t)b;
-            ctx->op_bytes += (int64_t)b;
-        }
         op->vals32 = p;
         op->bytes += cnt * 4;
         ctx->op_bytes += cnt * 4;
     }
     if (op->kind == 1 && op->diag32 == nullptr) {
         void* p = nullptr;
-        if (cudaMalloc(&p, (size_t)op->n * 4 + 64) != cudaSuccess)
+        if (rc_device_alloc(ctx, &p, (size_t)op->n * 4 + 64) != cudaSuccess)
             return rc_fail(ctx, RC_ERR_NOMEM, "cudaMalloc failed for FP32 stencil diagonal");
         cvt_f64_f32_kernel<<<4 * kB200Sms, 256, 0, ctx->stream>>>(op->diag64, (float*)p, op->n);
         ctx->launches++;

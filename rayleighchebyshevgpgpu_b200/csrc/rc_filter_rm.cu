@@ -148,7 +148,7 @@ struct StageOffsets {
     int n = 0;
     int64_t off[rc_op::kMaxOffsets] = {};
     int64_t max_row_nnz = 0;
-    const rc_op* op = nullptr;
+    rc_op* op = nullptr;
 };
 
 static bool stage_offsets(const rc_op* op, StageOffsets* so) {

@@ -151,10 +151,16 @@ struct rc_op {
     void* vals64 = nullptr;
     void* vals32 = nullptr;  // built lazily for the mixed-precision filter
     // 7-point structure: every row holds the diagonal and exactly its in-grid neighbours of a gx x gy x gz grid,
-    // columns ascending (0: not so). Then also the rows' weights, eight per row, for the tile kernels (rc_tile.cu).
+    // columns ascending (0: not so).
     int64_t gx = 0, gy = 0, gz = 0;
-    void* pack64 = nullptr;
-    void* pack32 = nullptr;
+    // Then the tile kernels may want the rows' weights, eight per row: tile_weights (rc_tile.cu) lays them out, FP64 [0]
+    // and FP32 [1], once the steps have moved pack_moved bytes of blocks without them. Not part of `bytes`, which the
+    // request server charges and refuses by: the server never lays them out.
+    std::atomic<void*> pack[2] = {};
+    int64_t pack_moved[2] = {0, 0};
+    int64_t pack_bytes = 0;
+    bool pack_refused = false;  // no memory was left: not asked for again
+    std::atomic<bool> pack_shared{false};  // another context (the server's) has read them
     // stencil
     int skind = 7;
     int64_t nx = 1, ny = 1, nz = 1;
@@ -198,6 +204,8 @@ cudaError_t allow_max_smem(const rc_ctx* ctx, K kernel) {
                                 (int)(ctx->smem_optin - fa.sharedSizeBytes));
 }
 
+// cudaMalloc that gives the operators' packed weights back before it fails.
+cudaError_t rc_device_alloc(rc_ctx* ctx, void** out, size_t bytes);
 // Scratch slot of at least `bytes` (contents not preserved on growth).
 rc_status rc_slot(rc_ctx* ctx, int slot, size_t bytes, void** out);
 // Free every scratch slot (stream-ordered when the context has a memory pool).
@@ -345,7 +353,7 @@ rc_status resid_norms(rc_ctx* ctx, int dtype, int64_t n, int64_t res_count, cons
 // res (device), and with R the row-major copy of R in the correction filter's storage (rc_corr_t or
 // rc_corr2_t, leading dimension corr_leading_dim(dtype, s)). One pass over Yrm.
 bool resid_supported(const rc_op* op, int64_t s);
-rc_status resid_block(rc_ctx* ctx, const rc_op* op, const void* Yrm, int64_t ld, int64_t s, const double* lam,
+rc_status resid_block(rc_ctx* ctx, rc_op* op, const void* Yrm, int64_t ld, int64_t s, const double* lam,
                       int64_t res_count, double* res, void* R, int64_t ldr);
 
 // Cholesky factor of Gram G (s x s) with diagonal scaling, shift on breakdown;

@@ -391,7 +391,7 @@ static rc_status resid_dispatch(rc_ctx* ctx, const rc_op* op, const T* Y, int64_
     return resid_ix<StencilRows<double, T, 5>, T>(ctx, pol, n, s, Y, ld, lam, res_count, res, R, ldr);
 }
 
-rc_status resid_block(rc_ctx* ctx, const rc_op* op, const void* Yrm, int64_t ld, int64_t s, const double* lam,
+rc_status resid_block(rc_ctx* ctx, rc_op* op, const void* Yrm, int64_t ld, int64_t s, const double* lam,
                       int64_t res_count, double* res, void* R, int64_t ldr) {
     if (!resid_supported(op, s)) return rc_fail(ctx, RC_ERR_UNSUPPORTED, "residual block: unsupported operator");
     if (res_count < 0 || res_count > s || ld != rm_leading_dim(op->dtype, P64, s) ||

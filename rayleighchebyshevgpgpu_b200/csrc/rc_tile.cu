@@ -555,18 +555,27 @@ __global__ void tile_pack_kernel(int64_t n, int nx, int ny, int nz, const int32_
     }
 }
 
+// A CSR operator's weights are laid out once its steps have moved this many bytes of blocks through the gather kernels.
+// A step loses 0.22 to 0.36 us per MB of its block (FP64 128^3 x 96, 1.6 GB: 1146 against 758 us; bfloat16, 0.4 GB: 347
+// against 242; FP64 48^3 x 96, 85 MB: 68 against 50), and laying the weights out takes 0.45 ms: cudaMalloc 0.4 at every
+// size from 1 MB on, the packing 0.05 per 134 MB. That is 1.2 to 2 GB of blocks; the line lies lower because most operators
+// see hundreds of steps, but above what a single call on a small one moves. Eight new operators of 8,000 to 216,000 rows:
+// their first batch of corrections 4.7 ms with weights for every grid from its creation on (and 2.9 ms more to create
+// them), 3.2 ms now; 48^3 rows x 24 columns 0.9 and 0.6 ms.
+constexpr int64_t kPackPerByte = 2, kPackBase = 256ll << 20;
+
 struct Structure {
     int kind = -1;
     int64_t nx = 0, ny = 0, nz = 0;
 };
-Structure structure(const rc_op* op, bool fp32) {
+Structure structure(const rc_ctx* ctx, const rc_op* op, bool fp32) {
     Structure S;
     if (op->kind == 1 && (op->skind == 7 || op->skind == 27)) {
         S.kind = op->skind == 7 ? TK_STENCIL7 : TK_STENCIL27;
         S.nx = op->nx;
         S.ny = op->ny;
         S.nz = op->nz;
-    } else if (op->kind == 0 && op->gx > 0 && (fp32 ? op->pack32 : op->pack64)) {
+    } else if (tile_rows(ctx, op, fp32)) {
         S.kind = TK_CSR7;
         S.nx = op->gx;
         S.ny = op->gy;
@@ -685,7 +694,7 @@ bool tile_launch(rc_ctx* ctx, const TileArgs& A, const TileMaps& M, const TileSt
 
 bool tile_supported(const rc_ctx* ctx, const rc_op* op, TileType type, int64_t ld, bool resid) {
     if (!ctx->tile) return false;
-    const Structure S = structure(op, type == TT_BF16 || type == TT_BF16C);
+    const Structure S = structure(ctx, op, type == TT_BF16 || type == TT_BF16C);
     if (S.kind < 0 || (op->dtype == RC_COMPLEX128) != (type == TT_C128 || type == TT_BF16C)) return false;
     if (S.kind == TK_STENCIL27 && op->dtype == RC_COMPLEX128) return false;
     return ctx->tile > 1 || S.kind == TK_STENCIL27 ||
@@ -693,10 +702,10 @@ bool tile_supported(const rc_ctx* ctx, const rc_op* op, TileType type, int64_t l
 }
 
 template <class TS, class TC, class TM, bool SRC>
-static bool tile_step_t(rc_ctx* ctx, const rc_op* op, TileType type, int64_t ld, const void* x, const void* z, void* y,
+static bool tile_step_t(rc_ctx* ctx, rc_op* op, TileType type, int64_t ld, const void* x, const void* z, void* y,
                         double alpha, double beta, double gamma, const void* src, const float* sig) {
     const bool fp32 = sizeof(real_t<TC>) == 4;
-    const Structure st = structure(op, fp32);
+    const Structure st = structure(ctx, op, fp32);
     TileArgs A;
     unsigned grid;
     size_t smem;
@@ -704,6 +713,8 @@ static bool tile_step_t(rc_ctx* ctx, const rc_op* op, TileType type, int64_t ld,
     const int wb = st.kind == TK_CSR7 ? (int)sizeof(RowWeights<TC>) : 0;
     const int64_t words = ld * (int64_t)sizeof(TM) / 4;
     if (!tile_plan(ctx, st, type, (int)(words / 4), zops, wb, &A, &grid, &smem)) return false;
+    const void* weights = wb ? tile_weights(ctx, op, fp32, op->n * ld * (int64_t)sizeof(TM)) : nullptr;
+    if (wb && !weights) return false;
     A.ld = ld;
     A.has_z = z != nullptr;
     A.off = op->offdiag;
@@ -713,7 +724,7 @@ static bool tile_step_t(rc_ctx* ctx, const rc_op* op, TileType type, int64_t ld,
     bool ok = tile_map(&M.x, x, st, words, A.nseg * 4, A.tx + 2, A.ty + 2);
     if (z) ok = ok && tile_map(&M.z, z, st, words, A.nseg * 4, A.tx, A.ty);
     if (SRC) ok = ok && tile_map(&M.src, src, st, words, A.nseg * 4, A.tx, A.ty);
-    if (wb) ok = ok && tile_map(&M.co, fp32 ? op->pack32 : op->pack64, st, wb / 4, wb / 4, A.tx, A.ty);
+    if (wb) ok = ok && tile_map(&M.co, weights, st, wb / 4, wb / 4, A.tx, A.ty);
     if (!ok) return false;
     TileStep<TM, TC> S;
     S.y = (TM*)y;
@@ -728,7 +739,7 @@ static bool tile_step_t(rc_ctx* ctx, const rc_op* op, TileType type, int64_t ld,
     return tile_launch<TK_STENCIL7, TS, TC, TM, SRC, false>(ctx, A, M, S, Q, grid, smem);
 }
 
-bool tile_step(rc_ctx* ctx, const rc_op* op, TileType type, int64_t ld, const void* x, const void* z, void* y, double alpha,
+bool tile_step(rc_ctx* ctx, rc_op* op, TileType type, int64_t ld, const void* x, const void* z, void* y, double alpha,
                double beta, double gamma, const void* src, const float* sig) {
     if (((uintptr_t)x | (uintptr_t)z | (uintptr_t)y | (uintptr_t)src) % 16) return false;
     switch (type) {
@@ -746,30 +757,32 @@ bool tile_step(rc_ctx* ctx, const rc_op* op, TileType type, int64_t ld, const vo
 }
 
 template <class T>
-static bool tile_resid_t(rc_ctx* ctx, const rc_op* op, const void* Y, int64_t ld, TileResid Q, int64_t res_count,
+static bool tile_resid_t(rc_ctx* ctx, rc_op* op, const void* Y, int64_t ld, TileResid Q, int64_t res_count,
                          double** part, int64_t* parts, rc_status* status) {
-    const Structure st = structure(op, false);
+    const Structure st = structure(ctx, op, false);
     TileArgs A;
     unsigned grid;
     size_t smem;
     const int wb = st.kind == TK_CSR7 ? (int)sizeof(RowWeights<T>) : 0;
     const int64_t words = ld * (int64_t)sizeof(T) / 4;
     if (!tile_plan(ctx, st, IsComplex<T>::value ? TT_C128 : TT_F64, (int)(words / 4), 0, wb, &A, &grid, &smem)) return false;
-    A.ld = ld;
-    A.off = op->offdiag;
-    A.diag = op->diag64;
-    A.phase = op->phase64;
-    TileMaps M = {};
-    bool ok = tile_map(&M.x, Y, st, words, A.nseg * 4, A.tx + 2, A.ty + 2);
-    if (wb) ok = ok && tile_map(&M.co, op->pack64, st, wb / 4, wb / 4, A.tx, A.ty);
-    if (!ok) return false;
-    if (res_count > 0) {
+    if (res_count > 0) {  // (before the weights: an allocation that fails may take them back)
         void* p = nullptr;
         *status = rc_slot(ctx, S_RPART, (size_t)grid * res_count * sizeof(double), &p);
         if (*status != RC_OK) return true;
         Q.part = *part = (double*)p;
         *parts = grid;
     }
+    const void* weights = wb ? tile_weights(ctx, op, false, op->n * ld * (int64_t)sizeof(T)) : nullptr;
+    if (wb && !weights) return false;
+    A.ld = ld;
+    A.off = op->offdiag;
+    A.diag = op->diag64;
+    A.phase = op->phase64;
+    TileMaps M = {};
+    bool ok = tile_map(&M.x, Y, st, words, A.nseg * 4, A.tx + 2, A.ty + 2);
+    if (wb) ok = ok && tile_map(&M.co, weights, st, wb / 4, wb / 4, A.tx, A.ty);
+    if (!ok) return false;
     const TileStep<T, T> S = {};
     if (st.kind == TK_CSR7) return tile_launch<TK_CSR7, T, T, T, false, true>(ctx, A, M, S, Q, grid, smem);
     if constexpr (!IsComplex<T>::value)
@@ -777,7 +790,7 @@ static bool tile_resid_t(rc_ctx* ctx, const rc_op* op, const void* Y, int64_t ld
     return tile_launch<TK_STENCIL7, T, T, T, false, true>(ctx, A, M, S, Q, grid, smem);
 }
 
-bool tile_resid(rc_ctx* ctx, const rc_op* op, const void* Y, int64_t ld, int64_t s, const double* lam, int64_t res_count,
+bool tile_resid(rc_ctx* ctx, rc_op* op, const void* Y, int64_t ld, int64_t s, const double* lam, int64_t res_count,
                 void* R, int64_t ldr, double** part, int64_t* parts, rc_status* st) {
     *st = RC_OK;
     if ((uintptr_t)Y % 16 || (uintptr_t)R % 4) return false;
@@ -791,31 +804,68 @@ bool tile_resid(rc_ctx* ctx, const rc_op* op, const void* Y, int64_t ld, int64_t
                                       : tile_resid_t<double>(ctx, op, Y, ld, Q, res_count, part, parts, st);
 }
 
-rc_status tile_pack(rc_ctx* ctx, const rc_op* op, bool fp32, const void* vals, void** out, size_t* bytes) {
+bool tile_rows(const rc_ctx* ctx, const rc_op* op, bool fp32) {
+    if (op->kind != 0 || op->gx <= 0) return false;
+    // only the operator's own context lays them out (a context belongs to one thread at a time), outside the server
+    return op->pack[fp32].load() || (ctx == op->ctx && !ctx->serve && !op->pack_refused);
+}
+
+const void* tile_weights(rc_ctx* ctx, rc_op* op, bool fp32, int64_t bytes) {
+    if (!tile_rows(ctx, op, fp32)) return nullptr;
+    if (ctx != op->ctx) op->pack_shared.store(true);  // before the pointer is read: tile_weights_release
+    if (const void* p = op->pack[fp32].load()) return p;
+    if (ctx != op->ctx) return nullptr;
     const bool cplx = op->dtype == RC_COMPLEX128;
-    *bytes = (size_t)op->n * 8 * elem_bytes(op->dtype, fp32 ? P32 : P64);
-    if (cudaMalloc(out, *bytes) != cudaSuccess) {
+    const int64_t size = op->n * 8 * (int64_t)elem_bytes(op->dtype, fp32 ? P32 : P64);
+    op->pack_moved[fp32] += bytes;
+    if (ctx->tile == 1 && op->pack_moved[fp32] < kPackPerByte * size + kPackBase) return nullptr;
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(ctx->stream, &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone)
+        return nullptr;
+    void* out = nullptr;
+    if (cudaMalloc(&out, (size_t)size) != cudaSuccess) {
         cudaGetLastError();
-        *out = nullptr;
-        return rc_fail(ctx, RC_ERR_NOMEM, "cudaMalloc for operator storage failed");
+        op->pack_refused = true;
+        return nullptr;
     }
     const unsigned g = (unsigned)std::min<int64_t>((op->n + 255) / 256, 16 * kB200Sms);
-    const int nx = (int)op->gx, ny = (int)op->gy, nz = (int)op->gz;
-    if (cplx && fp32)
-        tile_pack_kernel<float2><<<g, 256, 0, ctx->stream>>>(op->n, nx, ny, nz, op->rowptr, (const float2*)vals,
-                                                             (RowWeights<float2>*)*out);
-    else if (cplx)
-        tile_pack_kernel<double2><<<g, 256, 0, ctx->stream>>>(op->n, nx, ny, nz, op->rowptr, (const double2*)vals,
-                                                              (RowWeights<double2>*)*out);
-    else if (fp32)
-        tile_pack_kernel<float><<<g, 256, 0, ctx->stream>>>(op->n, nx, ny, nz, op->rowptr, (const float*)vals,
-                                                            (RowWeights<float>*)*out);
-    else
-        tile_pack_kernel<double><<<g, 256, 0, ctx->stream>>>(op->n, nx, ny, nz, op->rowptr, (const double*)vals,
-                                                             (RowWeights<double>*)*out);
+    auto pack = [&](auto v) {
+        using T = decltype(v);
+        tile_pack_kernel<T><<<g, 256, 0, ctx->stream>>>(op->n, (int)op->gx, (int)op->gy, (int)op->gz, op->rowptr,
+                                                        (const T*)(fp32 ? op->vals32 : op->vals64), (RowWeights<T>*)out);
+    };
+    if (fp32) cplx ? pack(float2()) : pack(float());
+    else cplx ? pack(double2()) : pack(double());
     ctx->launches++;
-    RC_CU(ctx, cudaGetLastError());
-    return RC_OK;
+    // complete before anyone sees them: the server's contexts read them on streams of their own
+    if (cudaGetLastError() != cudaSuccess || cudaStreamSynchronize(ctx->stream) != cudaSuccess) {
+        cudaFree(out);
+        return nullptr;
+    }
+    op->pack_bytes += size;
+    ctx->op_bytes += size;
+    op->pack[fp32].store(out);
+    return out;
+}
+
+bool tile_weights_release(rc_ctx* ctx) {
+    bool any = false;
+    for (rc_op* op : ctx->ops)
+        for (int k = 0; k < 2; ++k) {
+            void* p = op->pack[k].exchange(nullptr);
+            if (!p) continue;
+            if (op->pack_shared.load()) {  // another context's stream may be reading them
+                op->pack[k].store(p);
+                continue;
+            }
+            cudaStreamSynchronize(ctx->stream);
+            cudaFree(p);
+            const int64_t size = op->n * 8 * (int64_t)elem_bytes(op->dtype, k ? P32 : P64);
+            op->pack_bytes -= size;
+            ctx->op_bytes -= size;
+            op->pack_refused = any = true;
+        }
+    return any;
 }
 
 }  // namespace rcb
