@@ -31,6 +31,7 @@
 #include "rc_internal.h"
 #include "rc_rmstep.cuh"
 #include "rc_tile.h"
+#include "rc_tileplan.h"
 
 namespace rcb {
 
@@ -647,18 +648,7 @@ bool tile_plan(const rc_ctx* ctx, const Structure& S, TileType type, int slices,
     const int64_t columns = (int64_t)A.panels * A.ntx * A.nty;
     const int64_t ctas = std::max<int64_t>(1, ctx->sm_count / A.panels) * A.panels;
     if (columns * A.nz > INT32_MAX) return false;
-    // planes per unit: the fewest turns x planes read (two more of x per unit, about the cost of one plane)
-    double best = 1e300;
-    for (int k = 1; k <= A.nz; ++k) {
-        const int ml = (A.nz + k - 1) / k;
-        const int64_t units = columns * ((A.nz + ml - 1) / ml);
-        const double cost = (double)((units + ctas - 1) / ctas) * (ml + 1.2);
-        if (cost < best) {
-            best = cost;
-            A.ml = ml;
-        }
-        if (ml <= 4) break;
-    }
+    A.ml = tile_planes(A.nz, columns, ctas);
     A.nml = (A.nz + A.ml - 1) / A.ml;
     A.units = (int)(columns * A.nml);
     *grid = (unsigned)std::min<int64_t>(ctas, A.units);
