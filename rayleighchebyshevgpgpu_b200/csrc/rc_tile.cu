@@ -45,7 +45,7 @@ namespace {
 //             stencil 16 x 40 x 40 x 8 (3 MB) 93 -> 102, 32^3 x 53 (26 MB) 256 -> 203
 //   bfloat16  CSR 32^3 x 24 (1.5 MB) 131 -> 182, 48^3 x 53 (11 MB) 246 -> 189; stencil 48^3 x 24 (5 MB) 177 -> 156
 //   pairs     CSR 40^3 x 96 (23 MB) 412 -> 452; stencil 94 MB of c128 376 -> 396
-// 27 points: always (8^3, 24 columns: 303 -> 69).
+// 27 points: any block (8^3, 24 columns: 303 -> 69), where the plan pays (tile27_pays).
 constexpr int64_t tile_min_bytes(TileType t, bool csr, bool resid) {
     switch (t) {
         case TT_F64: return csr || resid ? 4ll << 20 : 32ll << 20;
@@ -648,7 +648,11 @@ bool tile_plan(const rc_ctx* ctx, const Structure& S, TileType type, int slices,
     const int64_t columns = (int64_t)A.panels * A.ntx * A.nty;
     const int64_t ctas = std::max<int64_t>(1, ctx->sm_count / A.panels) * A.panels;
     if (columns * A.nz > INT32_MAX) return false;
-    A.ml = tile_planes(A.nz, columns, ctas);
+    double planes = 0.0;
+    A.ml = tile_planes(A.nz, columns, ctas, &planes);
+    if (ctx->tile == 1 && S.kind == TK_STENCIL27 &&
+        !tile27_pays(type == TT_BF16, planes, 16.0 * slices * A.nx * A.ny * A.nz))
+        return false;
     A.nml = (A.nz + A.ml - 1) / A.ml;
     A.units = (int)(columns * A.nml);
     *grid = (unsigned)std::min<int64_t>(ctas, A.units);

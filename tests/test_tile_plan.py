@@ -30,7 +30,7 @@ int main() {
         const int64_t columns = (int64_t)std::exp(std::rand() / (double)RAND_MAX * std::log(5000.0));
         const int64_t c = ctas[std::rand() % 7];
         int tries = 0;
-        if (rcb::tile_planes(nz, columns, c, &tries) != one_by_one(nz, columns, c)) {
+        if (rcb::tile_planes(nz, columns, c, nullptr, &tries) != one_by_one(nz, columns, c)) {
             std::printf("nz %d columns %lld ctas %lld\n", nz, (long long)columns, (long long)c);
             return 1;
         }
@@ -39,7 +39,7 @@ int main() {
     for (int nz : {12000, 100000, 1000000})
         for (int64_t columns : {1, 2, 4, 40}) {
             int tries = 0;
-            rcb::tile_planes(nz, columns, 148, &tries);
+            rcb::tile_planes(nz, columns, 148, nullptr, &tries);
             most = tries > most ? tries : most;
         }
     std::printf("%d\n", most);
