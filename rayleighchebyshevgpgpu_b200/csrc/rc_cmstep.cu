@@ -36,6 +36,15 @@ constexpr size_t CM_MAX_SMEM = 224 * 1024;
 // Fewer than 8 columns leave no ring to fill.
 constexpr int64_t kCmMinBytes = 40ll << 20;
 
+// Largest waste of a plan, points copied and formed over those of the grid alone (narrow grids leave most of a tile
+// outside), for which the tiles are taken. Steps on 45 to 880 MB, gather -> tiles, us: CSR 130 x 70 x 90 x 24 (1.69) 130 -> 114,
+// 400 x 5 x 400 x 24 (2.0) 129 -> 137, 8 x 8 x 13,001 x 96 (2.5) 365 -> 560, 2 x 2 x 200,000 x 96 (21) 360 -> 3439; complex CSR
+// 6 x 6 x 25,000 x 56 (2.04) 744 -> 682, 3 x 5 x 50,000 x 24 (4.9) 292 -> 498; stencil 300 x 2 x 1300 x 8 (2.8) 77 -> 66,
+// 5 x 400 x 400 x 24 (3.8) 188 -> 261, 2 x 2 x 200,000 x 96 659 -> 3526; complex stencil 10 x 12 x 7000 x 24 (2.55) 242 -> 242,
+// 300 x 2 x 1300 x 24 (4.9) 228 -> 366; 5 points 17 x 50,001 x 8 (1.94) 78 -> 74, 2 x 600,000 x 96 (8.7) 942 -> 2220.
+template <class T>
+constexpr double cm_max_waste(bool csr) { return csr ? (sizeof(T) == 16 ? 2.5 : 1.9) : (sizeof(T) == 16 ? 2.6 : 3.0); }
+
 enum { CK_STENCIL7 = 0, CK_CSR7 = 1, CK_STENCIL5 = 2 };  // 5 points: the grid's y is the kernel's z
 template <class T>
 constexpr int cm_slots() { return sizeof(T) == 16 ? 4 : 6; }
@@ -257,7 +266,9 @@ bool cm_plan(const rc_ctx* ctx, int kind, int64_t nx, int64_t ny, int64_t nz, in
                 }
             }
         }
-    return best > 0.0;
+    if (best == 0.0) return false;
+    const double waste = (double)grid->x * (out->box + 2.0 * tile) / (3.0 * (double)nx * ny * nz);
+    return ctx->tile > 1 || waste <= cm_max_waste<T>(kind == CK_CSR7);
 }
 
 template <class T, int KIND>
