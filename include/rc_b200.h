@@ -75,6 +75,7 @@ rc_status rc_ctx_synchronize(rc_ctx* ctx);
 rc_status rc_ctx_launch_count(rc_ctx* ctx, int64_t* launches, int reset);
 /* A named counter of ctx since creation: "launches" (as rc_ctx_launch_count), "staged_launches"
  * (degree steps that ran with their operands staged in shared memory by asynchronous copies),
+ * "tile_launches" (operator steps and residual blocks formed from shared-memory tiles),
  * "pair_launches" (launches that ran two correction-filter degree steps in one pass),
  * "jacobi_sweeps" (Jacobi sweeps of the last rc_small_eigh call). */
 rc_status rc_ctx_counter(rc_ctx* ctx, const char* name, int64_t* value);

@@ -220,6 +220,7 @@ rc_status rc_ctx_counter(rc_ctx* ctx, const char* name, int64_t* value) {
     if (!ctx || !name || !value) return RC_ERR_INVALID;
     if (!std::strcmp(name, "launches")) *value = ctx->launches;
     else if (!std::strcmp(name, "staged_launches")) *value = ctx->staged_launches;
+    else if (!std::strcmp(name, "tile_launches")) *value = ctx->tile_launches;
     else if (!std::strcmp(name, "pair_launches")) *value = ctx->pair_launches;
     else if (!std::strcmp(name, "jacobi_sweeps")) *value = ctx->jacobi_sweeps;
     else return rc_fail(ctx, RC_ERR_INVALID, std::string("rc_ctx_counter: unknown counter ") + name);

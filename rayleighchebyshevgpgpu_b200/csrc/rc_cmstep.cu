@@ -283,6 +283,7 @@ rc_status cm_launch(rc_ctx* ctx, const rc_op* op, const StepArgs& a, T alpha, T 
                                                       alpha, beta, gamma, a.scale, (const RowWeights<T>*)weights,
                                                       op->diag64, op->offdiag, theta, lam, (int)res_count, part);
         ctx->launches++;
+        ctx->tile_launches++;
         RC_CU(ctx, cudaGetLastError());
         return RC_OK;
     };

@@ -109,6 +109,7 @@ struct rc_ctx {
     int corr_pair = 0;
     int64_t pair_launches = 0;
     int64_t staged_launches = 0;
+    int64_t tile_launches = 0;  // of the kernels of rc_tile.cu and rc_cmstep.cu
     // staged step shape: rows per chunk (multiple of 4) and pipeline stages; 0 = the largest that
     // fit. RCB200_STAGED_ROWS, RCB200_STAGED_STAGES.
     int staged_rows = 0;

@@ -593,10 +593,18 @@ constexpr int tile_elem(TileType t) { return t == TT_BF16 ? 2 : (t == TT_BF16C ?
 // 1076 -> 854; bfloat16 CSR 24 x 24 x 1000 x 24 (1.39, 288) 504 -> 453, the stencil 417 -> 444; 37 x 70 x 200 x 24 (1.36,
 // 96) 466 -> 511; pairs 18 x 11 x 4000 x 12 (2.03, 288) 701 -> 952. One slice a row of bfloat16 is too little for a TMA
 // box's lines (100 x 90 x 60 x 8: 213 -> 290).
-bool tile_pays(TileType type, bool csr, double waste, int threads, int nseg) {
+// Grids of few planes, and those whose units leave the last turn nearly empty, waste more than their edges: `total` is the
+// waste with the planes that the turns read. FP64 stencil 300 x 130 x 1 x 130 (total 2.7) 331 -> 464, x 2 x 53 (2.04)
+// 252 -> 274, x 4 x 53 (1.65) 533 -> 543; complex 300 x 130 x 1 x 53 (2.8) 297 -> 397, 300 x 2 x 130 x 53 (2.0) gains a
+// tenth; bfloat16 100 x 90 x 5 x 130 (2.9, 12 MB) 258 -> 293, the CSR rows 256 -> 281, smaller blocks (x 53, 5 MB) 181 -> 157.
+// (Not for steps without a second block, a filter's first and the residual, which were not measured there.)
+bool tile_pays(TileType type, bool csr, int zops, double waste, double total, double mbytes, int threads, int nseg) {
     const bool bf16 = type == TT_BF16 || type == TT_BF16C;
     if (bf16 && nseg < 2) return false;
     if (waste > (csr && type != TT_BF16C ? 1.45 : 1.3)) return false;
+    if (zops > 0 &&
+        (type == TT_BF16 ? total > (csr ? 2.4 : 2.1) && mbytes > 10.0 : !csr && !bf16 && total > (type == TT_F64 ? 2.0 : 2.4)))
+        return false;
     return threads >= (csr && !bf16 ? 160 : (type == TT_C128 ? 256 : 192));
 }
 
@@ -633,9 +641,6 @@ bool tile_plan(const rc_ctx* ctx, const Structure& S, TileType type, int slices,
             }
         }
     if (!A.tx) return false;
-    if (ctx->tile == 1 && S.kind != TK_STENCIL27 &&
-        !tile_pays(type, S.kind == TK_CSR7, least / ((double)A.nx * A.ny * (2.0 + zops)), A.tx * A.ty / R * A.nseg, A.nseg))
-        return false;
     A.xbytes = up(A.nseg * 16 * (A.tx + 2) * (A.ty + 2));
     A.zbytes = up(A.nseg * 16 * A.tx * A.ty);
     A.cbytes = up(wbytes * A.tx * A.ty);
@@ -650,9 +655,14 @@ bool tile_plan(const rc_ctx* ctx, const Structure& S, TileType type, int slices,
     if (columns * A.nz > INT32_MAX) return false;
     double planes = 0.0;
     A.ml = tile_planes(A.nz, columns, ctas, &planes);
-    if (ctx->tile == 1 && S.kind == TK_STENCIL27 &&
-        !tile27_pays(type == TT_BF16, planes, 16.0 * slices * A.nx * A.ny * A.nz))
-        return false;
+    if (ctx->tile == 1) {
+        const double bytes = 16.0 * slices * A.nx * A.ny * A.nz, waste = least / ((double)A.nx * A.ny * (2.0 + zops));
+        if (!(S.kind == TK_STENCIL27 ? tile27_pays(type == TT_BF16, planes, bytes)
+                                     : tile_pays(type, S.kind == TK_CSR7, zops, waste,
+                                                 waste * planes * ctas / ((double)columns * A.nz), bytes / 1048576.0,
+                                                 A.tx * A.ty / R * A.nseg, A.nseg)))
+            return false;
+    }
     A.nml = (A.nz + A.ml - 1) / A.ml;
     A.units = (int)(columns * A.nml);
     *grid = (unsigned)std::min<int64_t>(ctas, A.units);
@@ -681,6 +691,7 @@ bool tile_launch(rc_ctx* ctx, const TileArgs& A, const TileMaps& M, const TileSt
     const int nt = A.tx * A.ty / tl_rows(KIND) * A.nseg;
     kern<<<grid, nt + 32, smem, ctx->stream>>>(A, M, S, Q);
     ctx->launches++;
+    ctx->tile_launches++;
     return true;
 }
 
