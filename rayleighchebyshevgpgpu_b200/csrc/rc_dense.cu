@@ -1050,6 +1050,10 @@ rc_status small_eigh_work(rc_ctx* ctx, int dtype, int64_t s, void* A, void* Q, d
         return RC_OK;
     }
     const int nthr = ctx->jacobi_threads > 0 ? ctx->jacobi_threads : RC_JACOBI_THREADS;
+    if (head > 48 * 1024) {  // a round's rotations: real from 3073, complex from 2458 rows
+        if (dtype == RC_COMPLEX128) RC_CU(ctx, allow_max_smem(ctx, jacobi_kernel<double2>));
+        else RC_CU(ctx, allow_max_smem(ctx, jacobi_kernel<double>));
+    }
     if (dtype == RC_COMPLEX128)
         jacobi_kernel<double2><<<1, nthr, head, ctx->stream>>>((int)s, (const double2*)A, (double2*)Q, evals, info,
                                                                (double2*)work, sweeps);
