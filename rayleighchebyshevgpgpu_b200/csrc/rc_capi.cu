@@ -163,6 +163,7 @@ rc_status rc_ctx_create(int device, rc_ctx** out) {
         const int t = std::atoi(v) / 32 * 32;
         c->jacobi_threads = t >= 64 && t <= 1024 ? t : 0;
     }
+    if (const char* v = std::getenv("RCB200_LOST_STAGES")) c->lost = std::atoi(v) != 0 ? 1 : 0;
     if (const char* v = std::getenv("RCB200_TILE")) c->tile = std::max(0, std::min(2, std::atoi(v)));
     if (const char* v = std::getenv("RCB200_RM_RR")) c->rm_rr = std::atoi(v) != 0 ? 1 : 0;
     if (const char* v = std::getenv("RCB200_GRAM_C")) c->gram_c = std::atoi(v) != 0 ? 1 : 0;

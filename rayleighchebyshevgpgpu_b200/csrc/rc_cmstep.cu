@@ -62,6 +62,7 @@ struct CmArgs {
     int hx;                        // the tile's first column in the box
     int px, py, box, slot;         // the box's pitches and size, and the ring's step, in points
     int s, cols;                   // columns, and columns per CTA
+    int lost;                      // rc_ctx::lost
 };
 
 template <class T, int KIND, bool RES, bool TMA>
@@ -149,12 +150,16 @@ cm_step_kernel(CmArgs A, const __grid_constant__ CUtensorMap map, const T* __res
     }
     int slot = 0;
     unsigned phase = 0;
-    bool ok = true;  // a wait that ran out: the rest of the block is not a number
+    bool ok = !TMA || !A.lost;  // a wait that ran out: the rest of the block is not a number
+    int landed = 0;  // columns waited for
     for (int c = c0; c < c1; ++c) {
         if constexpr (TMA) ok = ok && mbar_wait(smem_u32(full + slot), phase);
         else cp_async_wait<S - 2>();
         __syncthreads();
-        if (ok) issue(c + S - 1, slot == 0 ? S - 1 : slot - 1);  // into the slot of column c - 1
+        if (ok) {
+            issue(c + S - 1, slot == 0 ? S - 1 : slot - 1);  // into the slot of column c - 1
+            landed = c + 1 - c0;
+        }
         if (RES && warp == 0 && c > c0 && c - 1 < res_count) {
             double v = lane < CM_THREADS / 32 ? red[(c - 1) & 1][lane] : 0.0;
 #pragma unroll
@@ -221,6 +226,11 @@ cm_step_kernel(CmArgs A, const __grid_constant__ CUtensorMap map, const T* __res
             slot = 0;
             phase ^= 1;
         }
+    }
+    if constexpr (TMA) {  // columns that were not waited for land before the CTA ends
+        if (!ok && tid == 0)
+            for (int k = landed; k < min(c1 - c0, landed + S - 1); ++k)
+                if (!mbar_wait(smem_u32(full + k % S), (k / S) & 1)) break;
     }
     if (RES && c1 > c0 && c1 - 1 < res_count) {
         __syncthreads();
@@ -314,6 +324,7 @@ rc_status cm_step_t(rc_ctx* ctx, rc_op* op, const StepArgs& a, const double* lam
         const int box[4] = {A.px * (int)W, A.py, A.tz + 2, 1};
         if (!tma_map_words_4d(&map, a.x, dims, box, a.ldx * W)) return RC_OK;
     }
+    A.lost = ctx->lost;
     const CUtensorMap* mp = tma ? &map : nullptr;
     double* pt = nullptr;
     if (res_count > 0) {

@@ -85,6 +85,7 @@ struct GrArgs {
     int only_w;          // real, one set: X^T W
     int stages;
     int aligned;         // TMA; else 8-byte copies (column-major)
+    int lost;            // rc_ctx::lost
 };
 // X and W; with an odd leading dimension their even columns, then their odd ones.
 struct GrMaps {
@@ -106,12 +107,11 @@ __device__ __forceinline__ void gr_rows(const GrArgs& A, const double* ring, int
     const int stage = A.ops * G::OP;
     int b = 0;
     unsigned ph = 0;
-    bool ok = true;
+    bool ok = !A.lost;
+    if (!ok) slabs = 0;
     for (int64_t s = 0; s < slabs; ++s) {
-        if (!mbar_wait(full + 8 * b, ph)) {
-            ok = false;
-            break;
-        }
+        ok = mbar_wait_warp(full + 8 * b, ph);
+        if (!ok) break;
         const double* xs = ring + b * stage;
         const double* ys = xs + (useW ? G::OP : 0);
 #pragma unroll 1
@@ -138,7 +138,8 @@ __device__ __forceinline__ void gr_rows(const GrArgs& A, const double* ring, int
             ph ^= 1;
         }
     }
-    if (!ok) acc[0][0] = __longlong_as_double(0x7ff8000000000000ll);  // a slab that never landed: NaN to the caller
+    // a slab that never landed: NaN to the caller (selected at the stores: to set the sums cost kilobytes of spills)
+    const double nan = __longlong_as_double(0x7ff8000000000000ll);
     if (A.kg > 1) {  // the groups' sums, in order, through the ring (every slab has been read)
         constexpr int NP = (T8 + 1) / 2;
         asm volatile("bar.sync 1, %0;" ::"r"(warps * 32) : "memory");
@@ -146,7 +147,7 @@ __device__ __forceinline__ void gr_rows(const GrArgs& A, const double* ring, int
         const int cs = A.sets * NP * (T8 + 1) * 32;
         if (kgi > 0) {
 #pragma unroll
-            for (int t = 0; t < NT; ++t) cb[(kgi - 1) * cs + t * 32] = make_double2(acc[t][0], acc[t][1]);
+            for (int t = 0; t < NT; ++t) cb[(kgi - 1) * cs + t * 32] = ok ? make_double2(acc[t][0], acc[t][1]) : make_double2(nan, nan);
         }
         asm volatile("bar.sync 1, %0;" ::"r"(warps * 32) : "memory");
         if (kgi > 0) return;
@@ -167,7 +168,7 @@ __device__ __forceinline__ void gr_rows(const GrArgs& A, const double* ring, int
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
             const int col = 8 * j + gr_col<LAY>(2 * q + h);
-            if (row < A.m && col < A.m) P[row + (int64_t)col * A.m] = acc[t][h];
+            if (row < A.m && col < A.m) P[row + (int64_t)col * A.m] = ok ? acc[t][h] : nan;
         }
     }
 }
@@ -217,7 +218,7 @@ __global__ void __launch_bounds__(32 * (GR_WARPS + 1), T8 <= 6 ? 2 : 1) gram_dmm
     unsigned ph = 0;
     int64_t used = 0;
     for (int64_t s = 0; s < slabs; ++s) {
-        if (used >= A.stages && !mbar_wait(empty + 8 * b, ph ^ 1)) break;
+        if (used >= A.stages && (A.lost || !mbar_wait_warp(empty + 8 * b, ph ^ 1))) break;
         const uint32_t bar = full + 8 * b;
         double* st = grsm + b * stage;
         const int64_t r0 = r_begin + s * G::SD;
@@ -397,6 +398,7 @@ rc_status gram_dmma(rc_ctx* ctx, int dtype, int64_t n, int64_t m, const void* X,
     GrArgs A = {};
     A.n = n;
     A.m = (int)m;
+    A.lost = ctx->lost;
     A.X = (const double*)X;
     A.lx = cplx ? 2 * ldx : ldx;
     A.W = (const double*)W;

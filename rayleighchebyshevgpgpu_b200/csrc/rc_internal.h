@@ -100,6 +100,9 @@ struct rc_ctx {
     // Degree steps and residual blocks of 7- and 27-point operators from shared-memory tiles (rc_tile.cu): 1
     // (default: large blocks), 0 (never) or 2 (always), from RCB200_TILE.
     int tile = 1;
+    // 1: the kernels fed by a ring of stages (rc_dmma.cuh) take its first stage for lost, as after a wait that ran out:
+    // what their outputs are then can be looked at. From RCB200_LOST_STAGES.
+    int lost = 0;
     // Rayleigh-Ritz of the correction filter's output on row-major blocks (the filtered block and
     // W = A V formed row-major, no transposes): 1 (default) or 0, from RCB200_RM_RR.
     int rm_rr = 1;

@@ -73,6 +73,7 @@ struct TileArgs {
     int xslots, zslots, xbytes, zbytes, cbytes;
     int zops;                       // planes per z slot: x_{k-2} and / or the source block
     int has_z;
+    int lost;                       // rc_ctx::lost
     double off;                     // stencils: every neighbour's weight, the diagonal and (complex) the phases
     const void* diag;
     const void* phase;
@@ -165,6 +166,45 @@ struct TileVec {
     }
 };
 
+// What a CTA's product threads form, in every unit, set to NaN (after a plane that never landed). Called, not inlined,
+// where its registers would be taken from the steps' loops (27 points 192^3, 48 columns: a correction of 9 steps 7.91 ms
+// inlined, 7.83 called; CSR 128^3, 96 columns, 13 steps 5.10 and 5.15).
+template <int KIND, class TS, class TC, class TM, bool RESID>
+__device__ __forceinline__ void tile_poison(const TileArgs& A, TM* y, const TileResid& Q) {
+    constexpr int V = Slice<TS, TM>::V, TL_ROWS = tl_rows(KIND);
+    constexpr bool CPLX = IsComplex<TC>::value;
+    const double nan = __longlong_as_double(0x7ff8000000000000ll);
+    unsigned id;  // (read again: places kept for these loops would cost the others registers)
+    asm volatile("mov.u32 %0, %%tid.x;" : "=r"(id));
+    const int r = (int)id / A.nseg, sg = (int)id - r * A.nseg;
+    for (int u = blockIdx.x; u < A.units; u += gridDim.x) {
+        const Unit U = tile_unit(A, u);
+        const int gx = U.x0 + (r & (A.tx - 1)), gy = U.y0 + (r >> A.ltx) * TL_ROWS, slice = U.panel * A.nseg + sg;
+        const int nrow = slice < A.slices && gx < A.nx ? max(0, min(TL_ROWS, A.ny - gy)) : 0;
+        for (int m = U.m0; m < U.m1; ++m)
+            for (int k = 0; k < nrow; ++k) {
+                const int64_t i = gx + (int64_t)A.nx * (gy + k + (int64_t)A.ny * m), col = (int64_t)slice * V;
+                if constexpr (RESID) {
+                    if (!Q.R) continue;
+                    using TR = typename std::conditional<CPLX, rc_corr2_t, rc_corr_t>::type;
+                    void* R = (TR*)Q.R + i * Q.ldr + col;
+                    if constexpr (sizeof(rc_corr_t) == 2) *(__nv_bfloat162*)R = __floats2bfloat162_rn((float)nan, (float)nan);
+                    else *(float2*)R = make_float2((float)nan, (float)nan);
+                } else {
+                    Slice<TS, TM> bad;
+#pragma unroll
+                    for (int v = 0; v < V; ++v) bad.v[v] = s_from<TS>(nan, nan);
+                    stv<TS, TM>(y + i * A.ld + col, bad);
+                }
+            }
+    }
+}
+
+template <int KIND, class TS, class TC, class TM, bool RESID>
+__device__ __noinline__ void tile_poison_call(const TileArgs& A, TM* y, const TileResid& Q) {
+    tile_poison<KIND, TS, TC, TM, RESID>(A, y, Q);
+}
+
 template <int KIND, class TS, class TC, class TM, bool SRC, bool RESID>
 __global__ void __launch_bounds__(TL_THREADS + 32, 1)
 tile_kernel(TileArgs A, const __grid_constant__ TileMaps M, TileStep<TM, TC> S, TileResid Q) {
@@ -181,7 +221,9 @@ tile_kernel(TileArgs A, const __grid_constant__ TileMaps M, TileStep<TM, TC> S, 
     const int zslot = A.zops * A.zbytes + A.cbytes;
     unsigned char* xs0 = tls;
     unsigned char* zs0 = tls + A.xslots * A.xbytes;
+    __shared__ int lost;
     if (tid == 0) {
+        lost = 0;
         for (int s = 0; s < A.xslots; ++s) {
             mbar_init(xfull + 8 * s, 1);
             mbar_init(xempty + 8 * s, nt / 32);
@@ -203,7 +245,7 @@ tile_kernel(TileArgs A, const __grid_constant__ TileMaps M, TileStep<TM, TC> S, 
         int64_t nxl = 0, nzl = 0;
         bool ok = true;
         auto load_x = [&](const Unit& U, int m) {
-            if (nxl >= A.xslots && !mbar_wait(xempty + 8 * rx.slot, rx.ph ^ 1)) return false;
+            if (nxl >= A.xslots && (A.lost || !mbar_wait(xempty + 8 * rx.slot, rx.ph ^ 1))) return false;
             const uint32_t bar = xfull + 8 * rx.slot;
             mbar_arrive_tx(bar, xtx);
             tma_load_4d(smem_u32(xs0 + rx.slot * A.xbytes), &M.x, U.panel * cw, U.x0 - 1, U.y0 - 1, m, bar);
@@ -212,7 +254,7 @@ tile_kernel(TileArgs A, const __grid_constant__ TileMaps M, TileStep<TM, TC> S, 
             return true;
         };
         auto load_z = [&](const Unit& U, int m) {
-            if (nzl >= A.zslots && !mbar_wait(zempty + 8 * rz.slot, rz.ph ^ 1)) return false;
+            if (nzl >= A.zslots && (A.lost || !mbar_wait(zempty + 8 * rz.slot, rz.ph ^ 1))) return false;
             const uint32_t bar = zfull + 8 * rz.slot;
             unsigned char* d = zs0 + rz.slot * zslot;
             mbar_arrive_tx(bar, ztx);
@@ -255,7 +297,7 @@ tile_kernel(TileArgs A, const __grid_constant__ TileMaps M, TileStep<TM, TC> S, 
     double sq[RESID ? V : 1];
 #pragma unroll
     for (int v = 0; v < (RESID ? V : 1); ++v) sq[v] = 0.0;
-    bool ok = true;
+    bool ok = !A.lost;
     for (int u = blockIdx.x; u < A.units && ok; u += gridDim.x) {
         const Unit U = tile_unit(A, u);
         const int gx = U.x0 + lx, gy = U.y0 + ly;
@@ -359,7 +401,9 @@ tile_kernel(TileArgs A, const __grid_constant__ TileMaps M, TileStep<TM, TC> S, 
             ok = ok && mbar_wait(xfull + 8 * rx.slot, rx.ph);
             return smem_u32(xs0) + rx.slot * A.xbytes + xo;
         };
+        // (all lanes come here whether their waits ran out or not, and go on together)
         auto free_x = [&](int slot) {
+            ok = __all_sync(~0u, ok);
             __syncwarp();
             if (lane == 0) mbar_arrive(xempty + 8 * slot);
         };
@@ -371,6 +415,7 @@ tile_kernel(TileArgs A, const __grid_constant__ TileMaps M, TileStep<TM, TC> S, 
         };
         auto free_z = [&]() {
             if (!zring) return;
+            if constexpr (KIND == TK_STENCIL27) ok = __all_sync(~0u, ok);  // (7 points: with free_x after it)
             __syncwarp();
             if (lane == 0) mbar_arrive(zempty + 8 * rz.slot);
             rz.next(A.zslots);
@@ -448,6 +493,7 @@ tile_kernel(TileArgs A, const __grid_constant__ TileMaps M, TileStep<TM, TC> S, 
                 rx.next(A.xslots);
             }
             uint32_t pc = wait_x();
+            ok = __all_sync(~0u, ok);
             int sc = rx.slot;
             rx.next(A.xslots);
             for (int m = U.m0; m < U.m1 && ok; ++m) {
@@ -508,19 +554,16 @@ tile_kernel(TileArgs A, const __grid_constant__ TileMaps M, TileStep<TM, TC> S, 
             free_x(sc);
         }
     }
-    if constexpr (!RESID) {
-        // a plane that never landed: NaN to the caller
-        if (!ok) {
-            Slice<TS, TM> bad;
-#pragma unroll
-            for (int v = 0; v < V; ++v) bad.v[v] = s_from<TS>(__longlong_as_double(0x7ff8000000000000ll), 0.0);
-            stv<TS, TM>(S.y, bad);
-        }
-    } else if (Q.res_count > 0) {
+    if (!ok) {  // a plane that never landed
+        if constexpr (KIND == TK_CSR7) tile_poison<KIND, TS, TC, TM, RESID>(A, S.y, Q);
+        else tile_poison_call<KIND, TS, TC, TM, RESID>(A, S.y, Q);
+    }
+    if constexpr (RESID) {
+        if (Q.res_count < 1) return;
         // column sums over the CTA's points, rows in order (the panel is the same in all its units)
-        if (!ok) sq[0] = __longlong_as_double(0x7ff8000000000000ll);
+        if (!ok) lost = 1;
         asm volatile("bar.sync 1, %0;" ::"r"(nt) : "memory");
-        double* red = reinterpret_cast<double*>(tls);  // every slot has been read
+        double* red = reinterpret_cast<double*>(tls);  // every slot has been read (or the sums are NaN)
         const int pw = A.nseg * V, rows = nt / A.nseg;
 #pragma unroll
         for (int v = 0; v < V; ++v) red[row * pw + seg * V + v] = sq[v];
@@ -530,6 +573,7 @@ tile_kernel(TileArgs A, const __grid_constant__ TileMaps M, TileStep<TM, TC> S, 
             double t = 0.0;
             if (c >= c0 && c < c0 + pw)
                 for (int r = 0; r < rows; ++r) t += red[r * pw + c - c0];
+            if (lost && c >= c0 && c < c0 + pw) t = __longlong_as_double(0x7ff8000000000000ll);
             Q.part[(int64_t)blockIdx.x * Q.res_count + c] = t;
         }
     }
@@ -616,6 +660,7 @@ bool tile_plan(const rc_ctx* ctx, const Structure& S, TileType type, int slices,
     A.ny = (int)S.ny;
     A.nz = (int)S.nz;
     A.slices = slices;
+    A.lost = ctx->lost;
     const int seg_max = S.kind == TK_STENCIL27 ? TL_MAX_SEG27 : TL_MAX_SEG, R = tl_rows(S.kind);
     A.panels = (slices + seg_max - 1) / seg_max;
     A.nseg = (slices + A.panels - 1) / A.panels;

@@ -93,7 +93,7 @@ template <bool CPLX, bool RM, bool ODD, int CT, bool RES, bool TRI>
 __global__ void __launch_bounds__(RES && !RM ? 288 : 544, RES && !RM ? 2 : 1)
 xt_dmma_kernel(const __grid_constant__ XtMaps maps, int64_t n, int k, int nc, const double* X, int64_t ldx, const double* __restrict__ Tm, int64_t ldt,
                double* Y, int64_t ldy, double* Yrm, int64_t ldyr, double alpha, double beta, int rs, int cg,
-               int stages, bool xv16, int yal) {
+               int stages, bool xv16, int yal, int lost) {
     using G = XtGeo<CPLX>;
     constexpr int CW = CPLX ? 2 : 1;              // doubles per scalar
     extern __shared__ __align__(128) double xtsm[];
@@ -141,7 +141,7 @@ xt_dmma_kernel(const __grid_constant__ XtMaps maps, int64_t n, int k, int nc, co
             const int64_t r0 = t << lmt;
             const int valid = (int)min((int64_t)MT, rows - r0);
             for (int ks = 0; ks < nk; ++ks) {
-                if (used >= stages && !mbar_wait(empty + 8 * b, ph ^ 1)) {
+                if (used >= stages && (lost || !mbar_wait_warp(empty + 8 * b, ph ^ 1))) {
                     ok = false;
                     break;
                 }
@@ -206,13 +206,11 @@ xt_dmma_kernel(const __grid_constant__ XtMaps maps, int64_t n, int k, int nc, co
     for (int m = 0; m < 2; ++m)
 #pragma unroll
         for (int j = 0; j < CT; ++j) acc[m][j][0] = acc[m][j][1] = 0.0;
-    bool ok = true;
-    for (int64_t t = blockIdx.x; t < ntiles && ok; t += gridDim.x) {
-        for (int ks = 0; ks < nk; ++ks) {
-            if (!mbar_wait(full + 8 * b, ph)) {
-                ok = false;
-                break;
-            }
+    bool ok = !lost;
+    for (int64_t t = blockIdx.x; t < ntiles; t += gridDim.x) {
+        for (int ks = 0; ks < nk && ok; ++ks) {
+            ok = mbar_wait_warp(full + 8 * b, ph);
+            if (!ok) break;
             const double* xs = ring + b * stage;
             const double* tp = (RES ? xtsm + ks * 32 : xs + xsz) + (grp * 8 * CT + g) * tpitch + 2 * q;
             const int kn = RM ? k : min(G::KS, k - ks * G::KS);
@@ -314,8 +312,12 @@ xt_dmma_kernel(const __grid_constant__ XtMaps maps, int64_t n, int k, int nc, co
                 ph ^= 1;
             }
         }
-        // a stage that never landed poisons the rows, so that the failure reaches the caller
-        if (!ok) acc[0][0][0] = __longlong_as_double(0x7ff8000000000000ll);
+        // a stage that never landed: the warp's part of this tile and of all that follow is NaN
+        if (!ok) {
+#pragma unroll
+            for (int j = 0; j < CT; ++j)
+                acc[0][j][0] = acc[0][j][1] = acc[1][j][0] = acc[1][j][1] = __longlong_as_double(0x7ff8000000000000ll);
+        }
         // the tile's rows of Y: a lane's rows r, r + 1 of columns c, c + 1 per 8-column tile
         const int64_t r = (t << lmt) + slab * 16 + 2 * g;
         const bool two = r + 1 < rows;
@@ -439,7 +441,7 @@ rc_status xt_dmma(rc_ctx* ctx, int dtype, int64_t n, int64_t k, int64_t nc, cons
         RC_CU(ctx, allow_max_smem(ctx, kern));
         kern<<<grid, 32 * (rs * cg + 1), smem, ctx->stream>>>(maps, n, (int)k, (int)nc, (const double*)X, ldx,
                                                              (const double*)Tk, ldt, (double*)Y, ldy, Yrm, ldyr, alpha,
-                                                             beta, rs, cg, stages, xv16, yal);
+                                                             beta, rs, cg, stages, xv16, yal, ctx->lost);
         ctx->launches++;
         RC_CU(ctx, cudaGetLastError());
         return RC_OK;
