@@ -10,9 +10,9 @@
 // come from L2, about four times the block's bytes, and L2 is the bound. A box of 32 x 8 x 8 points brings 1.6 times.
 // The sums are formed in the gather kernels' order (the same bits).
 //
-// Measured, with the gather kernels' time and the HBM floor, us: CSR 128^3, 96 columns 588 (1170, 492); 7-point stencil
-// 573 (1700, 492), with an odd nx 750; complex 24 x 24 x 768, 192 columns 443 (874, 415); 5-point 2048 x 1024, 64
-// columns 382 (1063, 328). By cp.async alone the first took 758: its copies were 23 of the 68 % of L1's data cycles.
+// Measured, with the gather kernels' time and the HBM floor, us: CSR 128^3, 96 columns 588 (1170, 512); 7-point stencil
+// 573 (1700, 494), with an odd nx 750; complex 24 x 24 x 768, 192 columns 443 (874, 415); 5-point 2048 x 1024, 64
+// columns 382 (1063, 330). By cp.async alone the first took 758: its copies were 23 of the 68 % of L1's data cycles.
 //
 // RES: the column sums of |y - lam x|^2 beside it (Rayleigh-Ritz residuals, which would read both blocks again),
 // per tile, in a fixed order.
@@ -150,16 +150,19 @@ cm_step_kernel(CmArgs A, const __grid_constant__ CUtensorMap map, const T* __res
     }
     int slot = 0;
     unsigned phase = 0;
-    bool ok = !TMA || !A.lost;  // a wait that ran out: the rest of the block is not a number
-    int landed = 0;  // columns waited for
+    bool ok = true;  // a wait that ran out: the rest of the block is not a number
     for (int c = c0; c < c1; ++c) {
-        if constexpr (TMA) ok = ok && mbar_wait(smem_u32(full + slot), phase);
+        if constexpr (TMA) {
+            if (ok && (A.lost || !mbar_wait(smem_u32(full + slot), phase))) {
+                ok = false;
+                if (tid == 0)  // the columns under way land before the CTA ends
+                    for (int k = c - c0; k < min(c1 - c0, c - c0 + S - 1); ++k)
+                        if (!mbar_wait(smem_u32(full + k % S), (k / S) & 1)) break;
+            }
+        }
         else cp_async_wait<S - 2>();
         __syncthreads();
-        if (ok) {
-            issue(c + S - 1, slot == 0 ? S - 1 : slot - 1);  // into the slot of column c - 1
-            landed = c + 1 - c0;
-        }
+        if (ok) issue(c + S - 1, slot == 0 ? S - 1 : slot - 1);  // into the slot of column c - 1
         if (RES && warp == 0 && c > c0 && c - 1 < res_count) {
             double v = lane < CM_THREADS / 32 ? red[(c - 1) & 1][lane] : 0.0;
 #pragma unroll
@@ -226,11 +229,6 @@ cm_step_kernel(CmArgs A, const __grid_constant__ CUtensorMap map, const T* __res
             slot = 0;
             phase ^= 1;
         }
-    }
-    if constexpr (TMA) {  // columns that were not waited for land before the CTA ends
-        if (!ok && tid == 0)
-            for (int k = landed; k < min(c1 - c0, landed + S - 1); ++k)
-                if (!mbar_wait(smem_u32(full + k % S), (k / S) & 1)) break;
     }
     if (RES && c1 > c0 && c1 - 1 < res_count) {
         __syncthreads();

@@ -208,9 +208,11 @@ xt_dmma_kernel(const __grid_constant__ XtMaps maps, int64_t n, int k, int nc, co
         for (int j = 0; j < CT; ++j) acc[m][j][0] = acc[m][j][1] = 0.0;
     bool ok = !lost;
     for (int64_t t = blockIdx.x; t < ntiles; t += gridDim.x) {
-        for (int ks = 0; ks < nk && ok; ++ks) {
-            ok = mbar_wait_warp(full + 8 * b, ph);
-            if (!ok) break;
+        for (int ks = ok ? 0 : nk; ks < nk; ++ks) {
+            if (!mbar_wait_warp(full + 8 * b, ph)) {
+                ok = false;
+                break;
+            }
             const double* xs = ring + b * stage;
             const double* tp = (RES ? xtsm + ks * 32 : xs + xsz) + (grp * 8 * CT + g) * tpitch + 2 * q;
             const int kn = RM ? k : min(G::KS, k - ks * G::KS);
