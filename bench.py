@@ -443,10 +443,11 @@ def run_ours(args):
     # (info.time_filter_steps_ms, transposes excluded). Degree-1 filters (column-major path, at
     # most a few per solve) are counted in degree_steps but not timed, a < 0.1 % overstatement.
     nnz = ci.size
-    # (the steps read the rows' packed weights, eight to a row, in place of the CSR arrays)
+    # (the FP64 and correction steps read the rows' packed weights, eight to a row, in place of the CSR arrays)
+    b_csr32 = nnz * (4 + 4) + (P.n + 1) * 4
     b_a32 = P.n * 8 * 4
     b_a64 = P.n * 8 * 8
-    bytes_fp32_step = b_a32 + 3 * P.n * s * 4
+    bytes_fp32_step = b_csr32 + 3 * P.n * s * 4
     ceb = int(infos[-1].get("correction_element_bytes", 4) or 4)
     bytes_corr_step = b_a32 + 4 * P.n * s * ceb
     bytes_fp64_step = b_a64 + 3 * P.n * s * 8

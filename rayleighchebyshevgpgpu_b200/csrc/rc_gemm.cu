@@ -107,7 +107,7 @@ xt_mma_kernel(int64_t n, int k, int nc, const double* __restrict__ X, int64_t ld
         load_cols_async<XM_RT, V16>(st, XM_RP, X, ldx, k, r0, n, tid, NT);
         load_cols_async<XM_RT, V16>(st + k4 * XM_RP, XM_RP, W, ldw, k, r0, n, tid, NT);
     };
-    // two stages, one barrier per tile (as in gram_mma_kernel)
+    // two stages, one barrier per tile
     int buf = 0;
     int64_t t = blockIdx.x;
     if (t < ntiles) issue(t, 0);

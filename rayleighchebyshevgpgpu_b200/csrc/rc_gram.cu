@@ -26,7 +26,7 @@
 // kernels this one replaced (32x32 super-blocks of both triangles' diagonal blocks, cp.async by the product
 // warps; SIMT for wider real blocks): 10^6 x 96 314 us (596; with an odd leading dimension 307, 795 before),
 // 2x10^6 x 48 179 us (522), 2x10^6 x 24 85 us (200), 216,000 x 36 19 us (60), 500,000 x 192 753 us (2041),
-// complex 442,368 x 96 534 us (752), x 192 2.58 ms (2.99); the sum over chunks 7-11 us (22-76).
+// complex 442,368 x 96 534 us (752), X^H W x 192 2.22 ms (2.99); the sum over chunks 7-11 us (22-76).
 #include <algorithm>
 #include "rc_common.cuh"
 #include "rc_dmma.cuh"

@@ -53,9 +53,10 @@ struct rc_ctx {
     double* host_small = nullptr;
     size_t host_small_bytes = 0;
     // and for rc_small_eigh's matrices (its own: an operator callback may call it during a solve)
-    rcb::BatchRunner* batch_runner = nullptr;  // of rc_filter_correction_batch (rc_corrapi.cu), from its first call on
     void* host_eigh = nullptr;
     size_t host_eigh_bytes = 0;
+    // of rc_filter_correction_batch (rc_corrapi.cu), from its first call on
+    rcb::BatchRunner* batch_runner = nullptr;
     int sm_count = 148;
     size_t smem_optin = 232448;
     // operators created on this context; rc_ctx_destroy releases the ones still alive
@@ -88,8 +89,8 @@ struct rc_ctx {
     // takes more where fewer cannot hold the matrix only when 0; otherwise of the kernels with the working copies in
     // global memory (0 = 32; 1 = one CTA).
     int jacobi_ctas = 0;
-    // Threads per CTA of the Jacobi kernels in shared memory and of one CTA (0: by size), from RCB200_JACOBI_THREADS; jacobi_sweeps is
-    // the number of sweeps the last rc_small_eigh call ran.
+    // Threads per CTA of the cluster Jacobi (0: by size, at most 512) and of the one-CTA kernel (0: 1024), from
+    // RCB200_JACOBI_THREADS; jacobi_sweeps is the number of sweeps the last rc_small_eigh call ran.
     int jacobi_threads = 0;
     // whether 16-CTA clusters run here, real and complex kernel (-1: not asked yet)
     int jacobi16_r = -1, jacobi16_c = -1;
@@ -97,8 +98,8 @@ struct rc_ctx {
     // for the FP64 SIMT kernel, from RCB200_GRAM_C.
     int gram_c = 1;
     int64_t jacobi_sweeps = 0;
-    // Degree steps and residual blocks of 7- and 27-point operators from shared-memory tiles (rc_tile.cu): 1
-    // (default: large blocks), 0 (never) or 2 (always), from RCB200_TILE.
+    // Degree steps and residual blocks of grid operators from shared-memory tiles (rc_tile.cu, rc_cmstep.cu): 1
+    // (default: where they gain), 0 (never) or 2 (wherever they can), from RCB200_TILE.
     int tile = 1;
     // 1: the kernels fed by a ring of stages (rc_dmma.cuh) take its first stage for lost, as after a wait that ran out:
     // what their outputs are then can be looked at. From RCB200_LOST_STAGES.
@@ -346,10 +347,10 @@ rc_status xt_dmma(rc_ctx* ctx, int dtype, int64_t n, int64_t k, int64_t nc, cons
                   double* Yrm = nullptr, int64_t ldyr = 0, bool tri = false);
 
 // res[c] = ||W_c - lam_c V_c|| for c < res_count (device), column-major blocks (rc_resid.cu).
-// op_step, and into res the norms of y - lam x of the first res_count columns (one kernel where the tiles take it).
-rc_status op_step_norms(rc_ctx* ctx, rc_op* op, const StepArgs& st, int64_t res_count, const double* lam, double* res);
 rc_status resid_norms(rc_ctx* ctx, int dtype, int64_t n, int64_t res_count, const void* V, int64_t ldv, const void* W,
                       int64_t ldw, const double* lam, double* res);
+// op_step, and into res the norms of y - lam x of the first res_count columns (one kernel where the tiles take it).
+rc_status op_step_norms(rc_ctx* ctx, rc_op* op, const StepArgs& st, int64_t res_count, const double* lam, double* res);
 
 // Residual block of Ritz vectors on native operators (rc_resid.cu; real, or complex CSR and 5/7-point
 // stencils; s <= kCorrMaxCols): R = A Y - Y diag(lam) from the row-major FP64 (c128) copy Yrm of Y

@@ -25,7 +25,8 @@ constexpr int64_t kNoAllocMaxS = 128;                                      // la
 constexpr size_t kEsz = 16;                                                // complex double (the wider scalar)
 constexpr size_t kMat = (size_t)kNoAllocMaxS * kNoAllocMaxS * kEsz;       // staging for H and for Q
 constexpr size_t kEvals = (size_t)kNoAllocMaxS * sizeof(double) + 256;     // eigenvalues + sweep count
-constexpr size_t kWork = 3 * (size_t)kNoAllocMaxS * (kNoAllocMaxS + 1) * kEsz;  // Jacobi working copies (A twice, Q)
+constexpr size_t kWork = 3 * (size_t)kNoAllocMaxS * (kNoAllocMaxS + 1) * kEsz;  // Jacobi working copies (A
+// twice, Q): read only where RCB200_JACOBI_CTAS keeps the cluster too small for the matrix
 constexpr size_t kScratchBytes = 2 * kMat + kEvals + kWork;
 
 // Shared by every call on a device; calls whose work overlaps on the GPU race on it.

@@ -151,7 +151,9 @@ int64_t solve_footprint(const rc_op* op, const rc_solve_params& p, int sm_count)
     t += round_2m((8 * (int64_t)sm_count + 2) * sq * sq * esz);       // Gram partial sums
     t += round_2m(((n + 63) / 64) * sq * 8);                         // residual partial sums
     t += round_2m(3 * n * esz + sq * sq * esz + 4096);                // Lanczos vectors / small QR
-    t += round_2m(4 * sq * sq * esz + 1024) + round_2m(2 * (sq + 1) * (sq + 1) * esz + 4096);  // cholqr, Jacobi
+    // cholqr; Jacobi's working copies, or, where a cluster's shared memory holds them (real to 470, complex to 320
+    // columns), in their place the products' T in the stages' layout (S_XTP), which is smaller
+    t += round_2m(4 * sq * sq * esz + 1024) + round_2m(2 * (sq + 1) * (sq + 1) * esz + 4096);
     if (op->kind == 2) t += round_2m(n * ss * esz);                   // callback step scratch
     if (rcb::resid_supported(op, ss))                                 // row-major copy of the Ritz vectors
         t += round_2m(n * rcb::rm_leading_dim(op->dtype, P64, ss) * esz);

@@ -17,8 +17,9 @@
 // reads instead of 8 (27 points: 4.5 instead of 9), no address or bounds arithmetic per neighbour, and nothing
 // waits on DRAM but the producer. The sums are formed in the gather kernels' order (5- and 7-point: the same bits).
 //
-// Measured, against the gather kernels (time per step; HBM floor): CSR 128^3, 96 columns, bfloat16 347 -> 242 us (246),
-// FP64 1146 -> 758 (760); 27 points 192^3, 48 columns, bfloat16 992 -> 467 (415), FP64 residual block 2204 -> 1016;
+// Measured, against the gather kernels (time per step; its bytes at the measured copy rate, 6.55 TB/s): CSR 128^3, 96
+// columns, bfloat16 347 -> 242 us (256: 7 % of the bytes are still in L2 from the step before), FP64 1146 -> 758 (758);
+// 27 points 192^3, 48 columns, bfloat16 992 -> 467 (419), FP64 residual block 2204 -> 1016;
 // complex stencil, 884,736 rows x 192 columns, bfloat16 pairs 570 -> 482 (415), bound by instruction issue.
 //
 // Units (a panel of a tile over ml planes) are taken in turn by one CTA per SM, panels fastest, then x, y, z: the
