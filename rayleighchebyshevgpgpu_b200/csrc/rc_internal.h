@@ -165,7 +165,7 @@ struct rc_op {
     int64_t pack_moved[2] = {0, 0};
     int64_t pack_bytes = 0;
     bool pack_refused = false;  // no memory was left: not asked for again
-    std::atomic<bool> pack_shared{false};  // another context (the server's) has read them
+    std::atomic<bool> pack_shared{false};  // another context (the server's) or a captured graph reads them: kept
     // stencil
     int skind = 7;
     int64_t nx = 1, ny = 1, nz = 1;

@@ -861,18 +861,26 @@ bool tile_rows(const rc_ctx* ctx, const rc_op* op, bool fp32) {
     return op->pack[fp32].load() || (ctx == op->ctx && !ctx->serve && !op->pack_refused);
 }
 
+static bool capturing(const rc_ctx* ctx) {
+    cudaStreamCaptureStatus s = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(ctx->stream, &s) == cudaSuccess) return s != cudaStreamCaptureStatusNone;
+    cudaGetLastError();
+    return true;
+}
+
 const void* tile_weights(rc_ctx* ctx, rc_op* op, bool fp32, int64_t bytes) {
     if (!tile_rows(ctx, op, fp32)) return nullptr;
     if (ctx != op->ctx) op->pack_shared.store(true);  // before the pointer is read: tile_weights_release
-    if (const void* p = op->pack[fp32].load()) return p;
+    if (const void* p = op->pack[fp32].load()) {
+        if (ctx == op->ctx && !op->pack_shared.load() && capturing(ctx)) op->pack_shared.store(true);  // a graph keeps it
+        return p;
+    }
     if (ctx != op->ctx) return nullptr;
     const bool cplx = op->dtype == RC_COMPLEX128;
     const int64_t size = op->n * 8 * (int64_t)elem_bytes(op->dtype, fp32 ? P32 : P64);
     op->pack_moved[fp32] += bytes;
     if (ctx->tile == 1 && op->pack_moved[fp32] < kPackPerByte * size + kPackBase) return nullptr;
-    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(ctx->stream, &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone)
-        return nullptr;
+    if (capturing(ctx)) return nullptr;
     void* out = nullptr;
     if (cudaMalloc(&out, (size_t)size) != cudaSuccess) {
         cudaGetLastError();
@@ -905,7 +913,7 @@ bool tile_weights_release(rc_ctx* ctx) {
         for (int k = 0; k < 2; ++k) {
             void* p = op->pack[k].exchange(nullptr);
             if (!p) continue;
-            if (op->pack_shared.load()) {  // another context's stream may be reading them
+            if (op->pack_shared.load()) {  // another context's stream, or a captured graph, may be reading them
                 op->pack[k].store(p);
                 continue;
             }

@@ -26,8 +26,8 @@ struct RowWeights {
 // them out; and the weights, for a step on a block of `bytes` (null: not laid out, the step takes the gather kernels).
 bool tile_rows(const rc_ctx* ctx, const rc_op* op, bool fp32);
 const void* tile_weights(rc_ctx* ctx, rc_op* op, bool fp32, int64_t bytes);
-// Gives back the weights of this context's operators, which only save time (not those that another context has read):
-// whether there were any. For an allocation that failed.
+// Gives back the weights of this context's operators, which only save time (not those that another context or a
+// captured graph reads): whether there were any. For an allocation that failed.
 bool tile_weights_release(rc_ctx* ctx);
 // op_step of a column-major FP64 block from tiles in shared memory (rc_cmstep.cu): *done is false (nothing launched)
 // where the operator, the types or the size are not for it. res_count > 0: also the partial column sums of
