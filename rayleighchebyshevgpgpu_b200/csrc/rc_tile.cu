@@ -167,9 +167,10 @@ struct TileVec {
     }
 };
 
-// What a CTA's product threads form, in every unit, set to NaN (after a plane that never landed). Called, not inlined,
-// where its registers would be taken from the steps' loops (27 points 192^3, 48 columns: a correction of 9 steps 7.91 ms
-// inlined, 7.83 called; CSR 128^3, 96 columns, 13 steps 5.10 and 5.15).
+// What a CTA's product threads form, in every unit, set to NaN (after a plane that never landed). 27 points: called, not
+// inlined, for its registers would be taken from the loops (192^3, 48 columns, a correction of 9 steps: 7.78 ms inlined,
+// 7.70 called), and with its arguments by value: a reference to the kernel's parameters has every thread copy them to
+// local memory at its start (7-point filter 100 x 90 x 60 x 24, 14 steps: 931 us inlined, 959 so).
 template <int KIND, class TS, class TC, class TM, bool RESID>
 __device__ __forceinline__ void tile_poison(const TileArgs& A, TM* y, const TileResid& Q) {
     constexpr int V = Slice<TS, TM>::V, TL_ROWS = tl_rows(KIND);
@@ -202,7 +203,7 @@ __device__ __forceinline__ void tile_poison(const TileArgs& A, TM* y, const Tile
 }
 
 template <int KIND, class TS, class TC, class TM, bool RESID>
-__device__ __noinline__ void tile_poison_call(const TileArgs& A, TM* y, const TileResid& Q) {
+__device__ __noinline__ void tile_poison_call(TileArgs A, TM* y, TileResid Q) {
     tile_poison<KIND, TS, TC, TM, RESID>(A, y, Q);
 }
 
@@ -556,7 +557,7 @@ tile_kernel(TileArgs A, const __grid_constant__ TileMaps M, TileStep<TM, TC> S, 
         }
     }
     if (!ok) {  // a plane that never landed
-        if constexpr (KIND == TK_CSR7) tile_poison<KIND, TS, TC, TM, RESID>(A, S.y, Q);
+        if constexpr (KIND != TK_STENCIL27) tile_poison<KIND, TS, TC, TM, RESID>(A, S.y, Q);
         else tile_poison_call<KIND, TS, TC, TM, RESID>(A, S.y, Q);
     }
     if constexpr (RESID) {
