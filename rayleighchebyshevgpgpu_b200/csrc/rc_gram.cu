@@ -95,7 +95,7 @@ struct GrMaps {
 // The product warps' loop over the chunk, for tile rows W and T8 - 1 - W.
 template <int T8, int LAY, int W>
 __device__ __forceinline__ void gr_rows(const GrArgs& A, const double* ring, int64_t slabs, uint32_t full, uint32_t empty,
-                                        int set, int kgi, bool useW, bool im, int lane, double* comb, int warps) {
+                                        int set, int kgi, bool useW, bool im, int lane, double* comb, int warps, int* lost) {
     using G = GrGeo<T8, LAY>;
     constexpr int R1 = T8 - 1 - W;
     constexpr bool TWO = R1 > W;
@@ -138,19 +138,19 @@ __device__ __forceinline__ void gr_rows(const GrArgs& A, const double* ring, int
             ph ^= 1;
         }
     }
-    // a slab that never landed: NaN to the caller (selected at the stores: to set the sums cost kilobytes of spills)
-    const double nan = __longlong_as_double(0x7ff8000000000000ll);
     if (A.kg > 1) {  // the groups' sums, in order, through the ring (every slab has been read)
         constexpr int NP = (T8 + 1) / 2;
         asm volatile("bar.sync 1, %0;" ::"r"(warps * 32) : "memory");
+        if (!ok && lane == 0) *lost = 1;
         double2* cb = reinterpret_cast<double2*>(comb) + ((set * NP + W) * (T8 + 1)) * 32 + lane;
         const int cs = A.sets * NP * (T8 + 1) * 32;
         if (kgi > 0) {
 #pragma unroll
-            for (int t = 0; t < NT; ++t) cb[(kgi - 1) * cs + t * 32] = ok ? make_double2(acc[t][0], acc[t][1]) : make_double2(nan, nan);
+            for (int t = 0; t < NT; ++t) cb[(kgi - 1) * cs + t * 32] = make_double2(acc[t][0], acc[t][1]);
         }
         asm volatile("bar.sync 1, %0;" ::"r"(warps * 32) : "memory");
         if (kgi > 0) return;
+        ok = *lost == 0;  // (any group)
         for (int k = 1; k < A.kg; ++k) {
 #pragma unroll
             for (int t = 0; t < NT; ++t) {
@@ -168,18 +168,27 @@ __device__ __forceinline__ void gr_rows(const GrArgs& A, const double* ring, int
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
             const int col = 8 * j + gr_col<LAY>(2 * q + h);
-            if (row < A.m && col < A.m) P[row + (int64_t)col * A.m] = ok ? acc[t][h] : nan;
+            if (row < A.m && col < A.m) P[row + (int64_t)col * A.m] = acc[t][h];
         }
+    }
+    if (ok) return;
+    // a slab that never landed: the warp's tiles are NaN (written over them: to set or select the sums cost up to
+    // kilobytes of spills)
+    const double nan = __longlong_as_double(0x7ff8000000000000ll);
+    for (int k = 0; k <= (TWO ? 1 : 0); ++k) {
+        const int i = k ? R1 : W, row = 8 * i + gr_col<LAY>(g);
+        for (int col = 8 * i + q; col < A.m; col += 4)
+            if (row < A.m) P[row + (int64_t)col * A.m] = nan;
     }
 }
 
 template <int T8, int LAY, int W = 0>
 __device__ __forceinline__ void gr_dispatch(int w, const GrArgs& A, const double* ring, int64_t slabs, uint32_t full,
                                             uint32_t empty, int set, int kgi, bool useW, bool im, int lane,
-                                            double* comb, int warps) {
+                                            double* comb, int warps, int* lost) {
     if constexpr (W < (T8 + 1) / 2) {
-        if (w == W) gr_rows<T8, LAY, W>(A, ring, slabs, full, empty, set, kgi, useW, im, lane, comb, warps);
-        else gr_dispatch<T8, LAY, W + 1>(w, A, ring, slabs, full, empty, set, kgi, useW, im, lane, comb, warps);
+        if (w == W) gr_rows<T8, LAY, W>(A, ring, slabs, full, empty, set, kgi, useW, im, lane, comb, warps, lost);
+        else gr_dispatch<T8, LAY, W + 1>(w, A, ring, slabs, full, empty, set, kgi, useW, im, lane, comb, warps, lost);
     }
 }
 
@@ -188,11 +197,13 @@ __global__ void __launch_bounds__(32 * (GR_WARPS + 1), T8 <= 6 ? 2 : 1) gram_dmm
     using G = GrGeo<T8, LAY>;
     extern __shared__ __align__(128) double grsm[];
     __shared__ __align__(8) uint64_t bars[2 * GR_STAGES];
+    __shared__ int lost;  // a group's wait ran out
     constexpr int NP = (T8 + 1) / 2;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int warps = NP * A.sets * A.kg;
     const uint32_t full = smem_u32(bars), empty = full + 8 * GR_STAGES;
     if (threadIdx.x == 0) {
+        lost = 0;
         for (int s = 0; s < A.stages; ++s) {
             mbar_init(full + 8 * s, A.aligned ? 1 : 33);
             mbar_init(empty + 8 * s, warps);
@@ -209,7 +220,7 @@ __global__ void __launch_bounds__(32 * (GR_WARPS + 1), T8 <= 6 ? 2 : 1) gram_dmm
         const int w = warp % NP, h = warp / NP, set = h % A.sets, kgi = h / A.sets;
         const int gset = A.set0 * blockIdx.y + set;  // which product (real) or part (complex)
         const bool useW = A.cplx ? A.ops == 2 : (A.only_w || gset == 1);
-        gr_dispatch<T8, LAY>(w, A, grsm, slabs, full, empty, set, kgi, useW, A.cplx && gset == 1, lane, grsm, warps);
+        gr_dispatch<T8, LAY>(w, A, grsm, slabs, full, empty, set, kgi, useW, A.cplx && gset == 1, lane, grsm, warps, &lost);
         return;
     }
     // the producer
@@ -218,7 +229,7 @@ __global__ void __launch_bounds__(32 * (GR_WARPS + 1), T8 <= 6 ? 2 : 1) gram_dmm
     unsigned ph = 0;
     int64_t used = 0;
     for (int64_t s = 0; s < slabs; ++s) {
-        if (used >= A.stages && (A.lost || !mbar_wait_warp(empty + 8 * b, ph ^ 1))) break;
+        if (used >= A.stages && (A.lost || !mbar_wait(empty + 8 * b, ph ^ 1))) break;
         const uint32_t bar = full + 8 * b;
         double* st = grsm + b * stage;
         const int64_t r0 = r_begin + s * G::SD;

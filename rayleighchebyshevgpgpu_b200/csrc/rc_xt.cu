@@ -141,7 +141,7 @@ xt_dmma_kernel(const __grid_constant__ XtMaps maps, int64_t n, int k, int nc, co
             const int64_t r0 = t << lmt;
             const int valid = (int)min((int64_t)MT, rows - r0);
             for (int ks = 0; ks < nk; ++ks) {
-                if (used >= stages && (lost || !mbar_wait_warp(empty + 8 * b, ph ^ 1))) {
+                if (used >= stages && (lost || !mbar_wait(empty + 8 * b, ph ^ 1))) {
                     ok = false;
                     break;
                 }
